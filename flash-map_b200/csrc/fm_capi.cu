@@ -221,6 +221,10 @@ struct fm_table {
     Ctl* h_ctl = nullptr;    // pinned mirror for readbacks
     uint32_t last_rounds = 0;  // rounds of the last mutating call (statistics)
     std::atomic<uint64_t> len{0};
+    // What the host knows of the table's history since it was created or
+    // cleared: a remove may have left tombstones; an insert may have claimed
+    // one (false only where Ctl::tomb_claimed is known to be 0).
+    std::atomic<bool> tombs{false}, claimed{false};
     cudaStream_t stream = nullptr;  // mutating calls
     std::mutex mu;                  // serialises mutating calls and their scratch
     OpScratch sc{};
@@ -349,7 +353,11 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // no rounds: ops grouped by the first EMPTY slot after their home
             // (lone ops at once, each group in index order); ops the kernels
             // leave (no EMPTY slot anywhere, groups too large) run in rounds
-            e = fm::launch_rem_direct(v, sh, kk, m, t->sc, t->d_ctl, s);
+            // -- or, while no insert has claimed a tombstone, in one pass in
+            // any order
+            const bool any_order = !t->claimed.load() && t->mask < (uint64_t)fm::DIST_MASK;
+            e = any_order ? fm::launch_rem_take(v, sh, kk, m, t->d_ctl, s)
+                          : fm::launch_rem_direct(v, sh, kk, m, t->sc, t->d_ctl, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
@@ -468,7 +476,9 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
 int run_rounds(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t* d_v, uint64_t n, cudaStream_t s,
                uint64_t* out_count, bool* limit) {
     uint32_t bits = 0;
+    if (!insert) t->tombs = true;
     int rc = run_rounds_inner(t, insert, d_k, d_v, n, s, out_count, &bits);
+    t->claimed = rc ? true : t->h_ctl->tomb_claimed != 0;  // the last readback is the call's end
     if (rc) {
         std::string msg = tl_err;
         recover(t, s);
@@ -798,6 +808,8 @@ int fm_clear(fm_table* t) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
     if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "clear", e);
     t->len.store(0);
+    t->tombs = false;
+    t->claimed = false;
     return FM_OK;
 }
 
@@ -919,6 +931,8 @@ int fm_load(fm_table* t, const uint32_t* flags, const void* keys, const void* va
     uint32_t persist[2] = {max_dist_of(flags, t->cap), 1u};
     if (e == cudaSuccess) e = cudaMemcpyAsync(&t->d_ctl->dmax, persist, 8, cudaMemcpyHostToDevice, t->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
+    t->tombs = true;
+    t->claimed = true;
     if (e != cudaSuccess) return cuda_fail(FM_ERR_TRANSFER, "load", e);
     t->len.store(len);
     return FM_OK;
@@ -939,6 +953,8 @@ int fm_copy(fm_table* dst, const fm_table* src, void* stream) {
         e = cudaMemcpyAsync(dst->d_vals, src->d_vals, src->cap * src->vsz, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess)  // dmax, tomb_claimed
         e = cudaMemcpyAsync(&dst->d_ctl->dmax, &src->d_ctl->dmax, 8, cudaMemcpyDeviceToDevice, s);
+    dst->tombs = e != cudaSuccess || src->tombs.load();
+    dst->claimed = e != cudaSuccess || src->claimed.load();
     if (e != cudaSuccess) return cuda_fail(FM_ERR_TRANSFER, "copy", e);
     dst->len.store(src->len.load());
     return FM_OK;
@@ -1133,6 +1149,7 @@ extern "C" int fm_bulk_insert_device_noalloc(fm_table* t, const void* d_keys, co
     uint64_t added = 0;
     bool limit = false;
     rc = noalloc_rounds(t, (const uint8_t*)d_keys, (const uint8_t*)d_values, (uint32_t)n, s, base, &added, &limit);
+    t->claimed = rc ? true : t->h_ctl->tomb_claimed != 0;
     if (rc) {
         const std::string msg = tl_err;
         cudaMemsetAsync(t->d_seg_min, 0xFF, t->cap * 4, s);
@@ -2071,6 +2088,15 @@ int fm_batch_capture(fm_batch* b, void* stream) {
     return FM_OK;
 }
 
+// The batch's removes may leave tombstones and its inserts claim them (what a
+// run did is known on the device only).
+static void batch_note_history(fm_batch* b) {
+    for (const fm_op& o : b->ops)
+        if (o.kind == FM_OP_REMOVE) o.table->tombs = true;
+    for (const fm_op& o : b->ops)
+        if (o.kind == FM_OP_INSERT && o.table->tombs.load()) o.table->claimed = true;
+}
+
 int fm_batch_run(fm_batch* b, void* stream) {
     if (!b) return fail(FM_ERR_INVALID_ARG, "batch is NULL");
     if (b->pending) return fail(FM_ERR_INVALID_ARG, "batch still running: call fm_batch_wait first");
@@ -2078,6 +2104,7 @@ int fm_batch_run(fm_batch* b, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     // tables must not have host-side work in flight on their own streams
     for (fm_table* t : b->tables) cudaStreamSynchronize(t->stream);
+    batch_note_history(b);
     int rc;
     if (b->exec) {
         rc = b->qmode ? queue_fill(b) : batch_fill(b);

@@ -147,6 +147,9 @@ cudaError_t launch_ins_comp(const TableView& t, Shape sh, const uint8_t* keys, c
 // warp) are left in pend[1] for the rounds from round 1.
 cudaError_t launch_rem_direct(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, const OpScratch& sc,
                               Ctl* ctl, cudaStream_t s);
+// A whole remove call of n0 ops on a table with Ctl::tomb_claimed 0 and fewer
+// than 2^28 slots: the ops commute, one kernel, nothing left over.
+cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, cudaStream_t s);
 // The same with the op count read from Ctl::n0 (nmax bounds it and sizes the
 // grids) and no host step after it: a call that found no EMPTY slot lists
 // every op in pend[1], so the rounds from round 1 complete the call either way.

@@ -536,10 +536,60 @@ void rounds_shape(const TableView& t, const uint8_t* keys, uint32_t n0, uint32_t
 // RX_BMAX ops leaves its ops to them (pend[1], Ctl::npend[1]).  Every
 // registration and list word is idle again when the five kernels end.
 
+// ---- removes of a table whose tombstones no insert has reused ---------------
+//
+// While no insert has claimed a TOMBSTONE since the table was cleared
+// (Ctl::tomb_claimed 0), the Robin Hood order holds: inserts only ever filled
+// EMPTY slots and raised stored distances, so every slot on the way from a
+// stored key's home to the key is OCCUPIED with a stored distance of at least
+// the probe depth there, or has become a TOMBSTONE, and no key is stored
+// twice.  So a probe finds its key, if it is stored at all, whatever other
+// slots the call's other removes have turned into tombstones, and finds
+// nothing otherwise: the ops commute, but for repeats of one key, of which
+// exactly one may count.  Each op probes on its own and exchanges the flag
+// word of its match for TOMBSTONE; the one that got the OCCUPIED word back
+// counts.  One pass over the ops, instead of grouping them by EMPTY slot
+// (find, exec, place, group and block passes).
+template <int KB>
+__device__ __forceinline__ uint32_t rx_take(const TableView& t, const uint8_t* keys, uint32_t j) {
+    RegKey<KB> key;
+    const uint64_t h = home_of<KB>(t, keys, j, key);
+    uint64_t stop;
+    const uint64_t x = rx_look<KB>(t, key, h, false, &stop);
+    return x != NONE64 && st_of(atomicExch(&t.flags[x], ST_TOMB)) == ST_OCC ? 1u : 0u;
+}
+
+// The whole call (the host knows that tomb_claimed is 0).  Bound by the
+// random reads of the probe (metadata sector, then key sector): a thread per
+// op with every thread of the SM resident keeps the most of them in flight.
+template <int KB>
+__global__ void __launch_bounds__(RBLOCK, 8) k_rx_take(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
+                                                       Ctl* ctl) {
+    __shared__ uint32_t s_tmp[RBLOCK / 32];
+    uint32_t removed = 0;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x)
+        removed += rx_take<KB>(t, keys, j);
+    block_add_count(ctl, removed, s_tmp);
+}
+
 template <int KB>
 __global__ void __launch_bounds__(RBLOCK) k_rx_find(TableView t, const uint8_t* __restrict__ keys, uint32_t n0_arg,
                                                     OpScratch sc, Ctl* ctl) {
+    __shared__ uint32_t s_tmp[RBLOCK / 32];
     const uint32_t n0 = n0_arg != CMP_N0_CTL ? n0_arg : *(volatile const uint32_t*)&ctl->n0;
+    if (n0_arg == CMP_N0_CTL && t.mask < (uint64_t)DIST_MASK && *(volatile const uint32_t*)&ctl->tomb_claimed == 0u) {
+        // a device-driven call: the table's history is known here only; the
+        // later passes find no op registered and no group
+        uint32_t removed = 0;
+        for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x) {
+            removed += rx_take<KB>(t, keys, j);
+            sc.op_slot[j] = NONE64;
+            sc.op_word[j] = IDLE;
+            sc.op_flag[j] = 0;
+        }
+        block_add_count(ctl, removed, s_tmp);
+        return;
+    }
     bool no_empty = false;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x) {
         RegKey<KB> key;
@@ -826,6 +876,21 @@ cudaError_t launch_rem_direct(const TableView& t, Shape sh, const uint8_t* keys,
         case SHAPE_32_32: direct_shape<32>(t, keys, n0, n0, sc, ctl, s); break;
         default: direct_shape<0>(t, keys, n0, n0, sc, ctl, s); break;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, cudaStream_t s) {
+    KtScope kt(KC_REM_EXEC, s);
+    const unsigned g = grid_for(n0, 8);
+    switch (sh) {
+        case SHAPE_8_8:
+        case SHAPE_8_32: k_rx_take<8><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
+        case SHAPE_32_128:
+        case SHAPE_32_64:
+        case SHAPE_32_32: k_rx_take<32><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
+        default: k_rx_take<0><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
+    }
+    count_launches(1);
     return cudaGetLastError();
 }
 
