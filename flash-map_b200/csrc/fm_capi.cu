@@ -271,17 +271,28 @@ struct TimerScope {
     ~TimerScope() { tl_timer = prev; }
 };
 
-int ensure_scratch(fm_table* t, uint64_t n) {
-    if (t->sc.cap_ops >= n) return FM_OK;
+int ensure_scratch(fm_table* t, uint64_t n, bool merge = false) {
+    if (t->sc.cap_ops >= n && (!merge || t->sc.carry)) return FM_OK;
+    merge = merge || t->sc.carry;
+    n = std::max(n, t->sc.cap_ops);
     // pend[0], pend[1] (u32) | op_slot (u64) | op_word (u32) | op_flag (u8) | op_pt (PT_MAX u32) |
     // long_list (u32) per op, then the component buffer and the remove chunk summaries (per table)
     const uint64_t per_op = 4 + 4 + 8 + 4 + 1 + 4 * fm::PT_MAX + 4;
     const uint64_t want = n + n / 4 + 1024;
-    const size_t bytes = (size_t)(want * per_op + 9 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
+    size_t bytes = (size_t)(want * per_op + 10 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
     if (t->sc_base) cudaFree(t->sc_base);
     t->sc_base = nullptr;
     t->sc = OpScratch{};
-    cudaError_t e = dev_alloc((void**)&t->sc_base, bytes);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!fault_at(FM_FAULT_ALLOC)) {
+        if (merge && (e = cudaMalloc((void**)&t->sc_base, bytes + fm::mg_bytes(t->mask))) == cudaSuccess) {
+            bytes += fm::mg_bytes(t->mask);
+        } else {  // no room for the merge's words: the call runs without them
+            if (merge) cudaGetLastError();
+            merge = false;
+            e = cudaMalloc((void**)&t->sc_base, bytes);
+        }
+    }
     if (e != cudaSuccess) return cuda_fail(FM_ERR_GPU_ALLOC, "scratch allocation", e);
     uint8_t* p = t->sc_base;
     auto carve = [&](size_t b) {
@@ -298,6 +309,7 @@ int ensure_scratch(fm_table* t, uint64_t n) {
     t->sc.long_list = (uint32_t*)carve(want * 4);
     t->sc.comp = carve(fm::cmp_bytes(t->mask));
     t->sc.rsum = (uint32_t*)carve(4 * fm::rsum_words(t->mask));
+    if (merge) t->sc.carry = (uint32_t*)carve(fm::mg_bytes(t->mask));
     t->sc.cap_ops = want;
     t->sc_bytes = bytes;
     // op_word doubles as the insert inflow bound: idle value 0xFFFFFFFF.
@@ -329,6 +341,19 @@ void recover(fm_table* t, cudaStream_t s) {
     cudaStreamSynchronize(s);
 }
 
+// Whether an insert of n ops runs as a merge: a table without tombstones, and
+// a call large enough beside the table that passes over all its slots cost
+// less than per-op work, and a load below FM_DIRECT_LOAD after it (beyond,
+// the runs are long and carry more ops than the merge keeps).
+#ifndef FM_MERGE_RATIO
+#define FM_MERGE_RATIO 16
+#endif
+bool merge_wanted(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n) {
+    return sh != fm::SHAPE_GENERIC && !t->tombs.load() && t->cap >= fm::MG_MIN_SLOTS &&
+           t->mask < (uint64_t)fm::DIST_MASK && n <= fm::MG_MAX_OPS && n * FM_MERGE_RATIO >= t->cap &&
+           (double)(len + n) < FM_DIRECT_LOAD * (double)t->cap;
+}
+
 // The round driver shared by insert and remove.  Each pass launches two
 // grid-wide rounds and the single-block tail back to back, then reads the
 // control block once: a zero pending count for the next round means done.
@@ -338,7 +363,8 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
     uint64_t total = 0;
     *err_bits = 0;
     const fm::Shape sh = t->shape_for({d_k, d_v});
-    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK);
+    const bool merge = insert && merge_wanted(t, sh, t->len.load(), n < OP_CHUNK ? n : OP_CHUNK);
+    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK, merge);
     if (rc) return rc;
     fm::TableView v = t->view();
     for (uint64_t base = 0; base < n; base += OP_CHUNK) {
@@ -372,6 +398,23 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
                 continue;
             }
             e = fm::launch_rem_summary(v, t->sc, t->d_ctl, s);
+            if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "round setup", e);
+        }
+        if (merge && t->sc.carry && merge_wanted(t, sh, t->len.load() + total, m)) {
+            e = fm::launch_ins_merge(v, sh, kk, vv, m, t->sc, t->d_ctl, s);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
+            if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "merge insert", e);
+            if (!t->h_ctl->serial[0]) {
+                total += t->h_ctl->total_count();
+                t->last_rounds = 0;
+                continue;
+            }
+            // left undone before any record moved: the paths below run the call
+            e = cudaMemsetAsync(t->d_seg_min, 0xFF, t->cap * 4, s);
+            if (e == cudaSuccess) e = cudaMemsetAsync(t->d_seg_cnt, 0, t->cap * 4, s);
+            if (e == cudaSuccess) e = cudaMemsetAsync(t->d_ctl, 0, fm::CTL_CALL_BYTES, s);
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "round setup", e);
         }
         // a chunk that can take the table to FM_DIRECT_LOAD or beyond runs as

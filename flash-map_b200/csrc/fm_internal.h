@@ -39,7 +39,7 @@ struct Ctl {
     unsigned long long count_part[COUNT_PARTS][4];  // the same from grid kernels, [i][0] used
     // Persistent table facts (survive across calls, reset by clear):
     uint32_t dmax;           // largest probe distance ever stored since clear
-    uint32_t tomb_claimed;   // 1 once an insert reused a tombstone since clear
+    uint32_t tomb_claimed;   // TOMB_* bits since clear
     unsigned long long occupied;  // recount result
     __host__ __device__ unsigned long long total_count() const {
         unsigned long long s = count;
@@ -47,6 +47,8 @@ struct Ctl {
         return s;
     }
 };
+constexpr uint32_t TOMB_CLAIMED = 1u;  // an insert reused a tombstone
+constexpr uint32_t TOMB_MADE = 2u;     // a remove ran (it may have left tombstones)
 constexpr size_t CTL_CALL_BYTES = 96 + 32 * COUNT_PARTS;  // npend .. count_part
 static_assert(offsetof(Ctl, count_part) % 32 == 0, "count parts in their own sectors");
 static_assert(offsetof(Ctl, dmax) == CTL_CALL_BYTES, "Ctl layout");
@@ -73,6 +75,7 @@ struct OpScratch {
     uint8_t* comp;       // insert: component buffer (cmp_bytes of the table; null: none)
     uint32_t* rsum;      // remove: per 32-slot chunk, a metadata summary then the least mark
                          //   (rsum_words of the table; marks IDLE between calls; null: none)
+    uint32_t* carry;     // merging inserts: mg_bytes of the table (null: none)
     uint64_t cap_ops;
 };
 
@@ -89,6 +92,15 @@ __host__ __device__ inline uint64_t cmp_chunks(uint64_t mask) { return (mask + C
 __host__ __device__ inline uint64_t cmp_bytes(uint64_t mask) { return 256 + cmp_chunks(mask) * 32; }
 constexpr uint32_t CMP_N0_CTL = 0xFFFFFFFFu;
 constexpr int PT_MAX = 4;
+
+// Merging inserts (fm_merge.cu): c per slot, c per chunk of MG_CHUNK slots,
+// the chunks' functions.
+constexpr uint64_t MG_CHUNK = 1024;       // slots per block of the scan
+constexpr uint64_t MG_MOVE_CHUNK = 1024;  // slots per block of the moves
+constexpr uint64_t MG_SMALL_SLOTS = 4096; // tables up to this size: one block does everything
+constexpr uint64_t MG_MIN_SLOTS = 1024;
+constexpr uint64_t MG_MAX_OPS = 1ull << 30;
+inline uint64_t mg_bytes(uint64_t mask) { return (mask + 1) * 4 + (mask + 1) / MG_CHUNK * 12; }
 
 enum Shape { SHAPE_8_8 = 0, SHAPE_32_128, SHAPE_32_64, SHAPE_32_32, SHAPE_8_32, SHAPE_GENERIC };
 Shape pick_shape(uint32_t ksz, uint32_t vsz);
@@ -122,6 +134,13 @@ cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys,
 // launch_ins_comp at round 1 with CMP_N0_CTL completes the call either way.
 cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
                                   uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s);
+// A whole insert call of n0 ops merged into a table without tombstones
+// (compile-time record shapes, MG_MIN_SLOTS to 2^28 slots, OpScratch::carry).
+// On return (stream-ordered) Ctl::serial[0] set means that no record has
+// moved: seg_min and seg_cnt are to be set idle and the call run by another
+// path; otherwise every op is done.
+cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                             const OpScratch& sc, Ctl* ctl, cudaStream_t s);
 // Runs every remaining round starting at r in one block if the pending count
 // is at most TAIL_MAX; otherwise returns without touching anything.  With
 // handoff, rounds that stop progressing are left pending for the host

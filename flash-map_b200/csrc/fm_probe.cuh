@@ -42,11 +42,19 @@ __device__ __forceinline__ void get_query_thread(const TableView& t, const uint8
 }
 
 template <int KB>
+__device__ __forceinline__ uint64_t get_probe_key(const TableView& t, const RegKey<KB>& key, uint64_t h);
+
+template <int KB>
 __device__ __forceinline__ uint64_t get_probe_thread(const TableView& t, const uint8_t* __restrict__ qk) {
-    const uint64_t mask = t.mask;
     RegKey<KB> key;
     key.load(qk, KB);
-    const uint64_t h = key.hash(KB, t.hash_mode) & mask;
+    return get_probe_key<KB>(t, key, key.hash(KB, t.hash_mode) & t.mask);
+}
+
+// The same with the key in registers and its home.
+template <int KB>
+__device__ __forceinline__ uint64_t get_probe_key(const TableView& t, const RegKey<KB>& key, uint64_t h) {
+    const uint64_t mask = t.mask;
     uint64_t wb = h & ~7ull;
     uint64_t hit = NONE64;
     bool done = false;
@@ -185,6 +193,33 @@ __device__ __forceinline__ void get_queries_lockstep(const TableView& t, const u
             if (ov) v[i].store(ov + q * VB, VB);
             if (of) of[q] = hit[g + i] != NONE64 ? 1 : 0;
         }
+    }
+}
+
+// The winning update of a slot: the largest op index (seg_min idle is the
+// largest word).
+__device__ __forceinline__ uint32_t upd_code(uint32_t j) { return 0x7FFFFFFFu - j; }
+
+// Copies the values of a warp's ops (src of each lane, null: none) to their
+// places together, LPV lanes per value.
+template <int VB>
+__device__ __forceinline__ void warp_copy_values(const uint8_t* src, uint8_t* dst) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if constexpr (VB % 16 == 0) {
+        constexpr uint32_t LPV = VB / 16, VPR = 32 / LPV;
+        if (__ballot_sync(0xFFFFFFFFu, src != nullptr) == 0) return;
+#pragma unroll
+        for (uint32_t r = 0; r < LPV; r++) {
+            const uint32_t who = r * VPR + lane / LPV;
+            const uint64_t s = __shfl_sync(0xFFFFFFFFu, (unsigned long long)src, who);
+            const uint64_t d = __shfl_sync(0xFFFFFFFFu, (unsigned long long)dst, who);
+            if (s)
+                reinterpret_cast<uint4*>(d)[lane % LPV] = __ldg(reinterpret_cast<const uint4*>(s) + lane % LPV);
+        }
+    } else if (src) {
+        RegVal<VB> v;
+        v.load_ro(src);
+        v.store(dst, VB);
     }
 }
 
