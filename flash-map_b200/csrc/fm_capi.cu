@@ -223,7 +223,7 @@ struct fm_table {
     std::atomic<uint64_t> len{0};
     // What the host knows of the table's history since it was created or
     // cleared: a remove may have left tombstones; an insert may have claimed
-    // one (false only where Ctl::tomb_claimed is known to be 0).
+    // one (false only where TOMB_CLAIMED is known not to be set).
     std::atomic<bool> tombs{false}, claimed{false};
     cudaStream_t stream = nullptr;  // mutating calls
     std::mutex mu;                  // serialises mutating calls and their scratch
@@ -521,7 +521,7 @@ int run_rounds(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t* d_v,
     uint32_t bits = 0;
     if (!insert) t->tombs = true;
     int rc = run_rounds_inner(t, insert, d_k, d_v, n, s, out_count, &bits);
-    t->claimed = rc ? true : t->h_ctl->tomb_claimed != 0;  // the last readback is the call's end
+    t->claimed = rc ? true : (t->h_ctl->tomb_claimed & fm::TOMB_CLAIMED) != 0;  // the last readback is the call's end
     if (rc) {
         std::string msg = tl_err;
         recover(t, s);
@@ -971,7 +971,7 @@ int fm_load(fm_table* t, const uint32_t* flags, const void* keys, const void* va
         e = cudaMemcpyAsync(t->d_vals, values, t->cap * t->vsz, cudaMemcpyHostToDevice, t->stream);
     // dmax bounds every stored distance; the history of a loaded table is
     // unknown, so tombstone reuse is assumed.
-    uint32_t persist[2] = {max_dist_of(flags, t->cap), 1u};
+    uint32_t persist[2] = {max_dist_of(flags, t->cap), fm::TOMB_CLAIMED | fm::TOMB_MADE};
     if (e == cudaSuccess) e = cudaMemcpyAsync(&t->d_ctl->dmax, persist, 8, cudaMemcpyHostToDevice, t->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
     t->tombs = true;
@@ -1192,7 +1192,7 @@ extern "C" int fm_bulk_insert_device_noalloc(fm_table* t, const void* d_keys, co
     uint64_t added = 0;
     bool limit = false;
     rc = noalloc_rounds(t, (const uint8_t*)d_keys, (const uint8_t*)d_values, (uint32_t)n, s, base, &added, &limit);
-    t->claimed = rc ? true : t->h_ctl->tomb_claimed != 0;
+    t->claimed = rc ? true : (t->h_ctl->tomb_claimed & fm::TOMB_CLAIMED) != 0;
     if (rc) {
         const std::string msg = tl_err;
         cudaMemsetAsync(t->d_seg_min, 0xFF, t->cap * 4, s);

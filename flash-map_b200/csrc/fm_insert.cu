@@ -623,7 +623,8 @@ __device__ __forceinline__ void publish_rare(Ctl* ctl, uint32_t maxd, bool tomb,
     limit = __any_sync(0xFFFFFFFFu, limit);
     if ((threadIdx.x & 31u) == 0) {
         if (maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, maxd);
-        if (tomb && !*(volatile uint32_t*)&ctl->tomb_claimed) ctl->tomb_claimed = 1u;
+        if (tomb && !(*(volatile uint32_t*)&ctl->tomb_claimed & TOMB_CLAIMED))
+            atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
         if (limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
     }
 }
@@ -1483,7 +1484,7 @@ __device__ __forceinline__ void ins_tail_body(const TableView& t, const uint8_t*
     __syncthreads();
     if (a.claimed) atomicAdd(&ctl->count, (unsigned long long)a.claimed);
     if (a.maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, a.maxd);
-    if (a.tomb) ctl->tomb_claimed = 1u;
+    if (a.tomb) atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
     if (a.limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1527,7 +1528,7 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_ins_serial(TableView t, cons
     __syncthreads();
     if (a.claimed) atomicAdd(&ctl->count, (unsigned long long)a.claimed);
     if (a.maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, a.maxd);
-    if (a.tomb) ctl->tomb_claimed = 1u;
+    if (a.tomb) atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
     if (a.limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1954,7 +1955,7 @@ __global__ void __launch_bounds__(CMP_EXEC_THREADS, 2) k_ins_comp(TableView t, c
     }
     if (a.claimed) atomicAdd(&ctl->count, (unsigned long long)a.claimed);
     if (a.maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, a.maxd);
-    if (a.tomb) ctl->tomb_claimed = 1u;
+    if (a.tomb) atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
     if (a.limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctl->npend[r & 1] = 0;
@@ -2010,8 +2011,9 @@ __global__ void __launch_bounds__(RBLOCK) k_cmp_clean(TableView t, OpScratch sc)
 constexpr uint32_t DX_ABS = 0x80000000u;   // seg_cnt: the free slot is in an earlier slot's component
 constexpr uint32_t DX_CNT = 0x7FFFFFFFu;
 constexpr uint32_t DX_ROOT = 0x80000000u;  // warp-pass list entry: a component's leader
+constexpr uint64_t DX_UPDATE = 1ull << 63; // op_slot: an update of that slot (tables without tombstones)
 #ifndef FM_DX_LCH
-#define FM_DX_LCH 4
+#define FM_DX_LCH 8
 #endif
 #ifndef FM_DX_LTRIPS
 #define FM_DX_LTRIPS 4
@@ -2039,6 +2041,15 @@ __device__ __forceinline__ void dx_let_next() {
 #if FM_DX_PDL
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #endif
+}
+
+// Whether the table has never held a tombstone since it was cleared: then no
+// key is stored twice, an op whose key is stored before the call stays an
+// update whatever the others do, and updates move nothing, so they are told
+// apart in the find pass and written before the exec pass (the last op on
+// each key), and only new keys go through the components.
+__device__ __forceinline__ bool dx_clean(const TableView& t, const Ctl* ctl) {
+    return t.mask >= 7 && t.mask < (uint64_t)DIST_MASK && *(volatile const uint32_t*)&ctl->tomb_claimed == 0u;
 }
 
 // First free slot at or after unwrapped position a, looking at no more than
@@ -2073,11 +2084,22 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_find(TableView t, const uint8_t* 
                                                     OpScratch sc, Ctl* ctl) {
     dx_let_next();
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
+    const bool clean = dx_clean(t, ctl);
     bool no_free = false;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x) {
         RegKey<KB> key;
         key.load(keys + (uint64_t)j * KB, KB);
         const uint64_t h = key.hash(KB, t.hash_mode) & t.mask;
+        if (clean) {
+            const uint64_t x = get_probe_key<KB>(t, key, h);
+            if (x != NONE64) {  // an update of slot x: the last op on it wins
+                sc.op_slot[j] = x | DX_UPDATE;
+                sc.op_word[j] = IDLE;
+                sc.op_flag[j] = 0;
+                atomicMin(&t.seg_min[x], upd_code(j));
+                continue;
+            }
+        }
         const uint64_t F = find_free_from(t, h);
         sc.op_slot[j] = F;
         sc.op_pt[(uint64_t)j * PT_MAX] = (uint32_t)h;  // the exec pass starts from it
@@ -2095,13 +2117,32 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_find(TableView t, const uint8_t* 
     if (no_free) ctl->serial[0] = 1u;
 }
 
-__global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, uint32_t n0_arg, OpScratch sc, Ctl* ctl) {
+template <int VB>
+__global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, const uint8_t* __restrict__ vals, uint32_t n0_arg,
+                                                    OpScratch sc, Ctl* ctl) {
     dx_wait_prev();
     dx_let_next();
-    if (*(volatile uint32_t*)&ctl->serial[0]) return;  // every op goes to the component path
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x) {
-        if (!sc.op_flag[j]) continue;
+    const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;  // every op goes to the component path, later
+    const bool clean = dx_clean(t, ctl);
+    const uint32_t iters = grid_iters(n0);
+    for (uint32_t it = 0; it < iters; it++) {  // warp-uniform trip count
+        const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x + it * gridDim.x * blockDim.x;
+        if (clean) {  // updates: nothing of the table moves before this pass ends
+            const uint8_t* src = nullptr;
+            uint8_t* dst = nullptr;
+            const uint64_t at = j < n0 ? sc.op_slot[j] : 0;
+            if (at != NONE64 && (at & DX_UPDATE)) {
+                const uint64_t x = at & ~DX_UPDATE;
+                if (t.seg_min[x] == upd_code(j)) {  // the others find another op's word, or idle
+                    src = vals + (uint64_t)j * VB;
+                    dst = t.vals + x * VB;
+                    t.seg_min[x] = IDLE;
+                }
+            }
+            warp_copy_values<VB>(src, dst);
+        }
+        if (serial || j >= n0 || !sc.op_flag[j]) continue;
         const uint64_t F = sc.op_slot[j];
         const uint32_t c = t.seg_cnt[F] & DX_CNT;
         if (c < 2) continue;
@@ -2131,50 +2172,15 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, uint32_t n0_arg
 
 // The thread path's per-thread lists (shared memory, one column per thread):
 // eviction slots and depths, possible-update slots and the evictions before
-// each.
+// each; and per warp the moves of its ops (lane << 8 | move).
 struct DxLaneSmem {
     uint32_t pos[DX_LCH][DX_THREADS];
     uint32_t dep[DX_LCH][DX_THREADS];
     uint32_t cpos[DX_LCMP][DX_THREADS];
-    uint32_t cst[DX_LCMP][DX_THREADS];
+    uint8_t cst[DX_LCMP][DX_THREADS];
+    uint16_t list[DX_THREADS / 32][32 * (DX_LCH + 1)];
 };
 
-// A record (key and value) held in registers for a move.
-template <int KB, int VB>
-struct DxRec {
-    RegKey<KB> k;
-    RegVal<VB> v;
-    __device__ __forceinline__ void load_in(const uint8_t* kp, const uint8_t* vp) {
-        k.load(kp, KB);
-        v.load_ro(vp);
-    }
-    __device__ __forceinline__ void load_slot(const TableView& t, uint64_t s, bool value_only) {
-        if (!value_only) k.load_table(t.keys + s * KB, KB);
-        v.load(t.vals + s * VB, VB);
-    }
-    __device__ __forceinline__ void store_slot(const TableView& t, uint64_t s, bool value_only) const {
-        if (!value_only) k.store(t.keys + s * KB, KB);
-        v.store(t.vals + s * VB, VB);
-    }
-};
-
-// One op alone at its free slot F (nothing of another op lies in [home, F]),
-// on one thread.  Every slot in [home, F) is occupied (F is the first free
-// slot at or after home), so the walk is in closed form: with H the home of
-// the carried entry (the op's home first), a resident whose home r exceeds H
-// is evicted (the carried entry takes its slot at depth position - H, and the
-// resident is carried on: H = r), one with r == H is a possible update, and F
-// takes the last carried entry.  The possible updates are compared first on
-// the keys' first 8 bytes, all in one round trip, and in full only where
-// those agree (the first equal key in walk order ends the walk in place);
-// then the records move highest first, DX_MB per round trip: move m writes
-// P_m (the m-th eviction slot; the end slot for the last) from P_(m-1) (the
-// new entry for m = 0), and a batch loads all its sources before it stores,
-// which keeps each slot's read before its write.  Returns 1 (claimed F), 0
-// (updated in place) or -1 with nothing written when the walk needs more than
-// DX_LTRIPS metadata reads, DX_LCH evictions or DX_LCMP possible updates, or
-// when the metadata does not show F as the first free slot.  Needs capacity
-// >= 8 and below 2^28 slots.
 // The first metadata window of a walk from home h (two aligned 8-slot
 // windows), loaded while the caller's other loads are in flight.
 struct DxWin {
@@ -2186,16 +2192,40 @@ struct DxWin {
     }
 };
 
-template <int KB, int VB>
-__device__ __noinline__ int dx_lane(const TableView& t, const RegKey<KB>& key, uint64_t h, uint64_t F,
-                                    const DxWin& w0, const uint8_t* kin, const uint8_t* vin, DxLaneSmem& sl,
-                                    ExecAcc& acc) {
-    constexpr int MB = (KB + VB) <= 16 ? 8 : ((KB + VB) <= 64 ? 4 : 2);  // moves per round trip
+// What one op alone at its free slot does (dx_plan): kind 1 claims F, 2
+// updates in place, 0 nothing to do, -1 too long for the thread path; k
+// evictions (their slots and depths in the thread's column), then the slot
+// `end` at depth `dep`.
+struct DxPlan {
+    int kind = 0;
+    uint32_t k = 0, end = 0, dep = 0;
+    bool tomb = false;
+};
+
+// One op alone at its free slot F (nothing of another op lies in [home, F]),
+// on one thread.  Every slot in [home, F) is occupied (F is the first free
+// slot at or after home), so the walk is in closed form: with H the home of
+// the carried entry (the op's home first), a resident whose home r exceeds H
+// is evicted (the carried entry takes its slot at depth position - H, and the
+// resident is carried on: H = r), one with r == H is a possible update, and F
+// takes the last carried entry.  The possible updates are compared on the
+// keys' first 8 bytes, all in one round trip, and in full only where those
+// agree (the first equal key in walk order ends the walk in place); with
+// `fresh` (the key is not stored, on a table where no key is stored twice)
+// there is nothing to compare.  Reads only.  -1 when the walk needs more than
+// DX_LTRIPS metadata reads, DX_LCH evictions or DX_LCMP possible updates, or
+// when the metadata does not show F as the first free slot.  Needs capacity
+// >= 8 and below 2^28 slots.
+template <int KB>
+__device__ __forceinline__ DxPlan dx_plan(const TableView& t, const RegKey<KB>& key, uint64_t h, uint64_t F,
+                                          const DxWin& w0, bool fresh, DxLaneSmem& sl) {
+    DxPlan p;
+    p.kind = -1;
     const uint64_t mask = t.mask;
     const uint32_t me = threadIdx.x;
     const uint64_t e = h + ((F - h) & mask);  // F, unwrapped
     const uint64_t wb = h & ~7ull;
-    if (e - wb >= 16ull * DX_LTRIPS) return -1;
+    if (e - wb >= 16ull * DX_LTRIPS) return p;
     uint32_t k = 0, nc = 0;
     long long H = (long long)h;
     bool end_tomb = false;
@@ -2210,31 +2240,31 @@ __device__ __noinline__ int dx_lane(const TableView& t, const RegKey<KB>& key, u
             const uint64_t pos = w + l;
             if (pos < h || pos > e) continue;
             if (pos == e) {
-                if (!is_free(f16[l])) return -1;  // not the free slot the find pass saw
+                if (!is_free(f16[l])) return p;  // not the free slot the find pass saw
                 end_tomb = st_of(f16[l]) == ST_TOMB;
                 continue;
             }
-            if (st_of(f16[l]) != ST_OCC) return -1;  // a free slot before F: likewise
+            if (st_of(f16[l]) != ST_OCC) return p;  // a free slot before F: likewise
             const long long r = (long long)pos - (long long)dist_of(f16[l]);
             if (r > H) {
-                if (k == (uint32_t)DX_LCH) return -1;
+                if (k == (uint32_t)DX_LCH) return p;
                 sl.pos[k][me] = (uint32_t)(pos & mask);
                 sl.dep[k][me] = (uint32_t)((long long)pos - H);
                 ++k;
                 H = r;
-            } else if (r == H) {
-                if (nc == (uint32_t)DX_LCMP) return -1;
+            } else if (r == H && !fresh) {
+                if (nc == (uint32_t)DX_LCMP) return p;
                 sl.cpos[nc][me] = (uint32_t)(pos & mask);
-                sl.cst[nc][me] = k;
+                sl.cst[nc][me] = (uint8_t)k;
                 ++nc;
             }
         }
     }
-    // possible updates: 8-byte prefixes of the resident and the carried keys
-    // in one round trip, full keys only where the prefixes agree
-    int kind = 1;
-    uint64_t end_slot = e & mask;
-    uint32_t kk = k;
+    p.kind = 1;
+    p.end = (uint32_t)(e & mask);
+    p.dep = (uint32_t)((long long)e - H);
+    p.k = k;
+    p.tomb = end_tomb;
     if (nc) {
         uint2 rp[DX_LCMP], cp[DX_LCMP];
         const uint2 kp = make_uint2(key.w[0], KB >= 8 ? key.w[1] : 0u);
@@ -2253,50 +2283,98 @@ __device__ __noinline__ int dx_lane(const TableView& t, const RegKey<KB>& key, u
                 if (q == c) agree = rp[q].x == cp[q].x && rp[q].y == cp[q].y;
             if (!agree) continue;
             const uint32_t st = sl.cst[c][me];
-            const uint64_t cs = sl.cpos[c][me];
+            const uint32_t cs = sl.cpos[c][me];
             RegKey<KB> ck;
             if (st) ck.load_table(t.keys + (uint64_t)sl.pos[st - 1][me] * KB, KB);
             else ck = key;
-            if (ck.eq(t.keys + cs * KB, KB)) {
-                kind = 2, end_slot = cs, kk = st;
+            if (ck.eq(t.keys + (uint64_t)cs * KB, KB)) {
+                p.kind = 2, p.end = cs, p.k = st, p.tomb = false;
                 break;
             }
         }
     }
-    // moves, highest first, MB per round trip
-    for (int top = (int)kk; top >= 0; top -= MB) {
-        DxRec<KB, VB> rec[MB];
+    return p;
+}
+
+// The moves that the plans of a warp's 32 ops ask for (op j of each lane):
+// move m of an op writes P_m (the m-th eviction slot; the end slot for m = k)
+// from P_(m-1) (the new entry for m = 0).  The warp lists them, each op's
+// highest first, and runs 32 at a time together, one 16-byte piece (8 for
+// records not of whole 16s) per lane and step, so that an instruction covers
+// whole records instead of one piece of 32 scattered ones.  A batch loads all
+// its records before it stores any, and later batches read only slots below
+// the ones stored, so each slot is read before it is written.  Ops of
+// different lanes touch disjoint slots.  Warp-uniform call.
+template <int KB, int VB>
+__device__ __forceinline__ void dx_moves(const TableView& t, const uint8_t* __restrict__ keys,
+                                         const uint8_t* __restrict__ vals, uint32_t j, const DxPlan& p,
+                                         DxLaneSmem& sl, ExecAcc& acc) {
+    using CO = ChunkOf<KB, VB>;
+    using Ch = typename CO::type;
+    constexpr int CK = CO::CK, NK = CO::NK, NP = CO::NC;
+    constexpr uint32_t NEW = 0x80000000u;      // the source is the new entry of an op
+    constexpr uint32_t VALUE_ONLY = 0xFFFFFFFFu;  // depth of an update in place
+    const uint32_t lane = threadIdx.x & 31u, wb = threadIdx.x & ~31u;
+    uint16_t* list = sl.list[threadIdx.x >> 5];
+    const uint32_t cnt = p.kind > 0 ? p.k + 1 : 0u;
+    uint32_t inc = cnt;
 #pragma unroll
-        for (int b = 0; b < MB; b++) {
-            const int m = top - b;
-            if (m < 0) continue;
-            const bool vo = kind == 2 && m == (int)kk;  // the update writes the value only
-            if (m == 0) rec[b].load_in(kin, vin);
-            else rec[b].load_slot(t, sl.pos[m - 1][me], vo);
-        }
-#pragma unroll
-        for (int b = 0; b < MB; b++) {
-            const int m = top - b;
-            if (m < 0) continue;
-            const bool vo = kind == 2 && m == (int)kk;
-            const uint64_t d = m < (int)kk ? (uint64_t)sl.pos[m][me] : end_slot;
-            rec[b].store_slot(t, d, vo);
-        }
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+        if ((int)lane >= d) inc += o;
     }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    for (uint32_t m = 0; m < cnt; m++) list[inc - cnt + m] = (uint16_t)(lane << 8 | (p.k - m));
+    __syncwarp();
+    const uint32_t dep_end = p.kind == 2 ? VALUE_ONLY : p.dep;
     uint32_t md = 0;
-    for (uint32_t i = 0; i < kk; i++) {
-        const uint32_t d = sl.dep[i][me];
-        t.flags[sl.pos[i][me]] = mk_flag(ST_OCC, d);
-        md = max(md, d);
+    for (uint32_t b = 0; b < total; b += 32) {
+        const uint32_t nb = min(32u, total - b);
+        const uint32_t code = lane < nb ? list[b + lane] : lane << 8;
+        const uint32_t ow = code >> 8, m = code & 255u;
+        const uint32_t ok = __shfl_sync(0xFFFFFFFFu, p.k, ow);
+        const uint32_t oe = __shfl_sync(0xFFFFFFFFu, p.end, ow);
+        const uint32_t od = __shfl_sync(0xFFFFFFFFu, dep_end, ow);
+        const uint32_t oj = __shfl_sync(0xFFFFFFFFu, j, ow);
+        uint32_t src = 0, dst = 0, dep = VALUE_ONLY;
+        if (lane < nb) {
+            src = m ? sl.pos[m - 1][wb + ow] : oj | NEW;
+            dst = m < ok ? sl.pos[m][wb + ow] : oe;
+            dep = m < ok ? sl.dep[m][wb + ow] : od;
+        }
+        Ch buf[NP];
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            const uint32_t g = lane + 32u * u, e = g / NP, c = g % NP;
+            const uint32_t s = __shfl_sync(0xFFFFFFFFu, src, e);
+            const uint32_t d = __shfl_sync(0xFFFFFFFFu, dep, e);
+            if (e >= nb || (d == VALUE_ONLY && c < (uint32_t)NK)) continue;
+            const uint64_t si = s & ~NEW;
+            const uint8_t* from = c < (uint32_t)NK ? (s & NEW ? keys : t.keys) + si * KB + c * CK
+                                                   : (s & NEW ? vals : t.vals) + si * VB + (c - NK) * CK;
+            buf[u] = *reinterpret_cast<const Ch*>(from);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            const uint32_t g = lane + 32u * u, e = g / NP, c = g % NP;
+            const uint64_t ds = __shfl_sync(0xFFFFFFFFu, dst, e);
+            const uint32_t d = __shfl_sync(0xFFFFFFFFu, dep, e);
+            if (e >= nb || (d == VALUE_ONLY && c < (uint32_t)NK)) continue;
+            uint8_t* to = c < (uint32_t)NK ? t.keys + ds * KB + c * CK : t.vals + ds * VB + (c - NK) * CK;
+            *reinterpret_cast<Ch*>(to) = buf[u];
+        }
+        if (dep != VALUE_ONLY) {
+            t.flags[dst] = mk_flag(ST_OCC, dep);
+            md = max(md, dep);
+        }
+        __syncwarp();
     }
-    if (kind == 1) {
-        const uint64_t d = (uint64_t)((long long)e - H);
-        t.flags[end_slot] = mk_flag(ST_OCC, d);
-        md = max(md, (uint32_t)d);
-        acc.tomb = acc.tomb || end_tomb;
+    if (p.kind == 1) {
+        acc.claimed += 1;
+        acc.tomb = acc.tomb || p.tomb;
     }
     acc.maxd = max(acc.maxd, md);
-    return kind == 1 ? 1 : 0;
 }
 
 // The exec pass: one thread per op (uniform trip count per warp, for the
@@ -2316,6 +2394,7 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
     const bool to_pend = n0_arg == CMP_N0_CTL;
     const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;
     const bool lanes_ok = t.mask >= 7 && t.mask < (uint64_t)DIST_MASK;
+    const bool fresh = dx_clean(t, ctl);  // updates are done: every op left has a key that is not stored
     ExecAcc a;
     // ops taken 32 at a time per warp from a counter (Ctl::exec_next, zero at
     // the start of the call): the grid is the resident blocks, and a warp that
@@ -2328,6 +2407,7 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
         const uint32_t j = j0 + (threadIdx.x & 31u);
         uint32_t item = 0;
         bool defer = false;
+        DxPlan p;
         if (j < n0 && serial && to_pend) sc.pend[1][atomicAdd(&ctl->npend[1], 1u)] = j;
         if (j < n0) {
             // independent loads together: free slot, home, key; then the
@@ -2335,8 +2415,8 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
             const uint64_t F = sc.op_slot[j];
             const uint64_t h = sc.op_pt[(uint64_t)j * PT_MAX];
             RegKey<KB> key;
-            key.load(keys + (uint64_t)j * KB, KB);
-            if (F != NONE64) {
+            if (!fresh) key.load(keys + (uint64_t)j * KB, KB);
+            if (F <= t.mask) {  // not an update, and a free slot
                 DxWin w0;
                 if (lanes_ok && !serial) w0.load(t, h & ~7ull);
                 const uint32_t w = t.seg_cnt[F];
@@ -2345,12 +2425,9 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
                     t.seg_cnt[F] = 0;
                     sc.op_word[j] = IDLE;
                 } else if (w == 1u) {  // alone at F, and F in no other op's component
-                    int c = -1;
-                    if (lanes_ok)
-                        c = dx_lane<KB, VB>(t, key, h, F, w0, keys + (uint64_t)j * KB, vals + (uint64_t)j * VB,
-                                            s_lane, a);
-                    if (c < 0) defer = true, item = j;
-                    else a.claimed += (uint32_t)c;
+                    p.kind = -1;
+                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, fresh, s_lane);
+                    if (p.kind < 0) defer = true, item = j;
                     t.seg_min[F] = IDLE;
                     t.seg_cnt[F] = 0;
                     sc.op_word[j] = IDLE;
@@ -2360,6 +2437,8 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
             }
         }
         append(sc.long_list, &ctl->nlong[0], item, defer);
+        __syncwarp();
+        dx_moves<KB, VB>(t, keys, vals, j, p, s_lane, a);
     }
     block_add_count(ctl, a.claimed, s_tmp);
     publish_rare(ctl, a.maxd, a.tomb, a.limit);
@@ -2712,6 +2791,7 @@ __device__ __noinline__ void q_begin(const QOp& o) {
             n0 = 0;
             st = STATUS_TABLE_FULL;
         }
+        if (o.kind == 2) atomicOr(&o.ctl->tomb_claimed, TOMB_MADE);
         o.ctl->n0 = n0;
         *o.status = st;
         *o.result = 0;
@@ -2794,6 +2874,7 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
         const uint32_t j = c * per + threadIdx.x + k * QTHREADS;
         uint32_t item = 0;
         bool defer = false;
+        DxPlan p;
         if (j < n0) {
             const uint64_t F = o.sc.op_slot[j];
             const uint64_t h = o.sc.op_pt[(uint64_t)j * PT_MAX];
@@ -2808,12 +2889,9 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
                     t.seg_cnt[F] = 0;
                     o.sc.op_word[j] = IDLE;
                 } else if (w == 1u) {
-                    int r = -1;
-                    if (lanes_ok)
-                        r = dx_lane<KB, VB>(t, key, h, F, w0, o.keys + (uint64_t)j * KB, o.vals + (uint64_t)j * VB,
-                                            sm.exec, a);
-                    if (r < 0) defer = true, item = j;
-                    else a.claimed += (uint32_t)r;
+                    p.kind = -1;
+                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, false, sm.exec);
+                    if (p.kind < 0) defer = true, item = j;
                     t.seg_min[F] = IDLE;
                     t.seg_cnt[F] = 0;
                     o.sc.op_word[j] = IDLE;
@@ -2823,6 +2901,8 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
             }
         }
         append(o.sc.long_list, &o.ctl->nlong[0], item, defer);
+        __syncwarp();
+        dx_moves<KB, VB>(t, o.keys, o.vals, j, p, sm.exec, a);
     }
     block_add_count(o.ctl, a.claimed, sm.tmp);
     publish_rare(o.ctl, a.maxd, a.tomb, a.limit);
@@ -2972,7 +3052,7 @@ __device__ __noinline__ void q_end(const QOp& o, QSmem& sm) {
             __syncthreads();
             if (a.claimed) atomicAdd(&o.ctl->count, (unsigned long long)a.claimed);
             if (a.maxd > *(volatile uint32_t*)&o.ctl->dmax) atomicMax(&o.ctl->dmax, a.maxd);
-            if (a.tomb) o.ctl->tomb_claimed = 1u;
+            if (a.tomb) atomicOr(&o.ctl->tomb_claimed, TOMB_CLAIMED);
             if (a.limit) atomicOr(&o.ctl->err, ERR_WALK_LIMIT);
         } else {
             // removes: mark, list in index order, then warp 0 runs them 32 at
@@ -3096,7 +3176,8 @@ __device__ __forceinline__ uint32_t grp_pending(const GroupOp* ops, uint32_t o, 
 
 __device__ __forceinline__ void grp_rare(Ctl* ctl, const ExecAcc& a) {
     if (a.maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, a.maxd);
-    if (a.tomb && !*(volatile uint32_t*)&ctl->tomb_claimed) ctl->tomb_claimed = 1u;
+    if (a.tomb && !(*(volatile uint32_t*)&ctl->tomb_claimed & TOMB_CLAIMED))
+        atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
     if (a.limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
 }
 
@@ -3216,7 +3297,7 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_grp_ins_serial(const GroupOp
     Ctl* ctl = g.ctl;
     if (a.claimed) atomicAdd(&ctl->count, (unsigned long long)a.claimed);
     if (a.maxd > *(volatile uint32_t*)&ctl->dmax) atomicMax(&ctl->dmax, a.maxd);
-    if (a.tomb) ctl->tomb_claimed = 1u;
+    if (a.tomb) atomicOr(&ctl->tomb_claimed, TOMB_CLAIMED);
     if (a.limit) atomicOr(&ctl->err, ERR_WALK_LIMIT);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -3427,7 +3508,7 @@ void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, 
         }
         {
             KtScope kt(KC_INS_WALK, s);
-            launch_dependent(k_dx_flow, g, RBLOCK, s, pdl, t, n0, sc, ctl);
+            launch_dependent(k_dx_flow<VB>, g, RBLOCK, s, pdl, t, vals, n0, sc, ctl);
         }
         {
             KtScope kt(KC_INS_EXEC, s);

@@ -539,7 +539,7 @@ void rounds_shape(const TableView& t, const uint8_t* keys, uint32_t n0, uint32_t
 // ---- removes of a table whose tombstones no insert has reused ---------------
 //
 // While no insert has claimed a TOMBSTONE since the table was cleared
-// (Ctl::tomb_claimed 0), the Robin Hood order holds: inserts only ever filled
+// (TOMB_CLAIMED not set), the Robin Hood order holds: inserts only ever filled
 // EMPTY slots and raised stored distances, so every slot on the way from a
 // stored key's home to the key is OCCUPIED with a stored distance of at least
 // the probe depth there, or has become a TOMBSTONE, and no key is stored
@@ -559,13 +559,14 @@ __device__ __forceinline__ uint32_t rx_take(const TableView& t, const uint8_t* k
     return x != NONE64 && st_of(atomicExch(&t.flags[x], ST_TOMB)) == ST_OCC ? 1u : 0u;
 }
 
-// The whole call (the host knows that tomb_claimed is 0).  Bound by the
+// The whole call (the host knows the table's history).  Bound by the
 // random reads of the probe (metadata sector, then key sector): a thread per
 // op with every thread of the SM resident keeps the most of them in flight.
 template <int KB>
 __global__ void __launch_bounds__(RBLOCK, 8) k_rx_take(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
                                                        Ctl* ctl) {
     __shared__ uint32_t s_tmp[RBLOCK / 32];
+    note_remove(ctl);
     uint32_t removed = 0;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x)
         removed += rx_take<KB>(t, keys, j);
@@ -577,7 +578,8 @@ __global__ void __launch_bounds__(RBLOCK) k_rx_find(TableView t, const uint8_t* 
                                                     OpScratch sc, Ctl* ctl) {
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     const uint32_t n0 = n0_arg != CMP_N0_CTL ? n0_arg : *(volatile const uint32_t*)&ctl->n0;
-    if (n0_arg == CMP_N0_CTL && t.mask < (uint64_t)DIST_MASK && *(volatile const uint32_t*)&ctl->tomb_claimed == 0u) {
+    note_remove(ctl);
+    if (n0_arg == CMP_N0_CTL && t.mask < (uint64_t)DIST_MASK && !(*(volatile const uint32_t*)&ctl->tomb_claimed & TOMB_CLAIMED)) {
         // a device-driven call: the table's history is known here only; the
         // later passes find no op registered and no group
         uint32_t removed = 0;

@@ -58,6 +58,12 @@ __device__ __forceinline__ uint32_t* pend_of(const OpScratch& sc, uint32_t r) {
     return (r & 1u) ? sc.pend[1] : sc.pend[0];
 }
 
+// A remove runs on the table (one thread of the grid says so).
+__device__ __forceinline__ void note_remove(Ctl* ctl) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !(*(volatile uint32_t*)&ctl->tomb_claimed & TOMB_MADE))
+        atomicOr(&ctl->tomb_claimed, TOMB_MADE);
+}
+
 // The ops of round r: round 0 is the identity over the call's n0 ops.
 struct RoundOps {
     const uint32_t* list;  // nullptr: identity
@@ -234,6 +240,7 @@ __global__ void k_grp_setup(const GroupOp* __restrict__ ops, int is_insert) {
             n0 = 0;
             st = STATUS_TABLE_FULL;
         }
+        if (!is_insert && n0) atomicOr(&g.ctl->tomb_claimed, TOMB_MADE);
         g.ctl->n0 = n0;
         *g.status = st;
         *g.result = 0;
