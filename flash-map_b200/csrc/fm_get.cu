@@ -182,6 +182,44 @@ __global__ void __launch_bounds__(BLOCK) k_get_thread(TableView t, const uint8_t
     }
 }
 
+// Run-time record sizes: a thread per query as k_get_thread, then the warp
+// moves its 32 values together in the widest pieces that the size and both
+// addresses allow.  One 8-lane tile per query (k_get<0, 0, 8>, which tables
+// of fewer than 8 slots keep) had an eighth of the probes in flight.
+__global__ void __launch_bounds__(BLOCK) k_get_any(TableView t, const uint8_t* __restrict__ qkeys, uint64_t n,
+                                                   uint8_t* __restrict__ out_vals, uint8_t* __restrict__ out_found) {
+    const uint32_t lane = threadIdx.x & 31u, vsz = t.vsz;
+    const uint32_t w = piece_of(t.vals, out_vals, vsz);  // every value's place is a multiple of it
+    const uint32_t per = vsz / w;
+    const uint64_t G = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += G) {
+        const uint64_t q = base + lane;
+        uint64_t hit = NONE64;
+        if (q < n) {
+            RegKey<0> key;
+            key.load(qkeys + q * t.ksz, t.ksz);
+            hit = get_probe_key<0, true>(t, key, key.hash(t.ksz, t.hash_mode) & t.mask);
+            if (out_found) out_found[q] = hit != NONE64 ? 1 : 0;
+        }
+        if (!out_vals) continue;
+        const uint32_t m = (uint32_t)(n - base < 32 ? n - base : 32);
+        for (uint32_t p0 = 0; p0 < m * per; p0 += 32) {  // warp-uniform
+            const uint32_t p = p0 + lane, who = p / per, at = (p - who * per) * w;
+            const uint64_t hs = __shfl_sync(0xFFFFFFFFu, hit, who & 31u);
+            if (who >= m) continue;
+            uint8_t* dst = out_vals + (base + who) * vsz + at;
+            const uint8_t* src = t.vals + hs * vsz + at;
+            if (w == 16)
+                *reinterpret_cast<uint4*>(dst) =
+                    hs != NONE64 ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(0u, 0u, 0u, 0u);
+            else if (w == 4)
+                *reinterpret_cast<uint32_t*>(dst) = hs != NONE64 ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
+            else
+                *dst = hs != NONE64 ? __ldg(src) : (uint8_t)0;
+        }
+    }
+}
+
 // Q queries per thread probed in lockstep (get_queries_lockstep): thread g
 // takes queries g, g + G, ..., g + (Q-1)G of each span of Q*G (G threads in
 // the grid), so a warp's key loads stay coalesced.
@@ -248,6 +286,14 @@ cudaError_t get_shape(const TableView& t, const uint8_t* q, uint64_t n, uint8_t*
                       cudaStream_t s) {
     int lanes = cfg.lanes;
     // one thread per query needs compile-time sizes and 8-slot windows
+    if constexpr (KB == 0) {
+        if (lanes == 1 && t.mask >= 7) {
+            KtScope kt(KC_GET, s);
+            k_get_any<<<grid_for(n, cfg.blocks_per_sm), BLOCK, 0, s>>>(t, q, n, ov, of);
+            g_launches += 1;
+            return cudaGetLastError();
+        }
+    }
     if (lanes == 1 && !(KB != 0 && VB != 0 && t.mask >= 7)) lanes = 8;
     switch (lanes) {
         case 1:
@@ -347,9 +393,7 @@ cudaError_t launch_get_cfg(const TableView& t, Shape sh, const uint8_t* q, uint6
 GetCfg tuned_get_cfg(Shape sh, double load) {
     const GetCfg c = g_tuned[sh][load_bucket(load)];
     if (c.lanes > 0 && c.blocks_per_sm > 0) return c;
-    GetCfg d;  // measured default on B200: one thread per query, 64 blocks per SM
-    if (sh == SHAPE_GENERIC) d.lanes = 8, d.blocks_per_sm = 16;
-    return d;
+    return GetCfg();  // measured default on B200: one thread per query, 64 blocks per SM
 }
 
 void set_tuned_get_cfg(Shape sh, int bucket, GetCfg cfg) {
@@ -358,9 +402,7 @@ void set_tuned_get_cfg(Shape sh, int bucket, GetCfg cfg) {
 
 cudaError_t launch_get(const TableView& t, Shape sh, const uint8_t* q, uint64_t n, uint8_t* ov, uint8_t* of,
                        cudaStream_t s) {
-    GetCfg cfg;
-    if (sh == SHAPE_GENERIC) cfg.lanes = 8, cfg.blocks_per_sm = 16;
-    return launch_get_cfg(t, sh, q, n, ov, of, cfg, s);
+    return launch_get_cfg(t, sh, q, n, ov, of, GetCfg(), s);
 }
 
 cudaError_t launch_grp_get(Shape sh, const GroupGet* ops, const uint64_t* prefix, uint32_t nops, uint64_t total,

@@ -81,7 +81,7 @@ __device__ __forceinline__ void mg_find(const TableView& t, const uint8_t* __res
     for (uint32_t j = me; j < n0; j += step) {
         RegKey<KB> key;
         const uint64_t h = home_of<KB>(t, keys, j, key);
-        const uint64_t x = get_probe_key<KB>(t, key, h);
+        const uint64_t x = get_probe_key<KB, true>(t, key, h);
         if (x != NONE64) {
             sc.op_slot[j] = x | MG_UPDATE;
             sc.op_flag[j] = 0;

@@ -41,26 +41,74 @@ __device__ __forceinline__ void get_query_thread(const TableView& t, const uint8
     if (of) *of = hit != NONE64 ? 1 : 0;
 }
 
-template <int KB>
+template <int KB, bool RO>
 __device__ __forceinline__ uint64_t get_probe_key(const TableView& t, const RegKey<KB>& key, uint64_t h);
 
 template <int KB>
 __device__ __forceinline__ uint64_t get_probe_thread(const TableView& t, const uint8_t* __restrict__ qk) {
     RegKey<KB> key;
     key.load(qk, KB);
-    return get_probe_key<KB>(t, key, key.hash(KB, t.hash_mode) & t.mask);
+    return get_probe_key<KB, true>(t, key, key.hash(KB, t.hash_mode) & t.mask);
 }
 
-// The same with the key in registers and its home.
-template <int KB>
+// An aligned window of eight metadata words against the words a key would
+// have there: slot l's is e0 + 16 l (depth << 4 | OCCUPIED).  cand: slots that
+// hold exactly it (the only ones that can hold the key); term: the probe ends
+// there -- EMPTY, or OCCUPIED with a smaller distance, which as words are both
+// smaller; the word TOMBSTONE is passed.  Slots before the home come out
+// arbitrary.  Depths below 2^28.
+__device__ __forceinline__ void window_masks(const uint4& a, const uint4& b, uint32_t e0, uint32_t& cand,
+                                             uint32_t& term) {
+    const uint32_t f8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    cand = 0, term = 0;
+#pragma unroll
+    for (int l = 0; l < 8; l++) {
+        const uint32_t e = e0 + 16u * l;
+        if (f8[l] == e) cand |= 1u << l;
+        if (f8[l] < e && f8[l] != ST_TOMB) term |= 1u << l;
+    }
+}
+
+// The same with the key in registers and its home.  RO: the table is not
+// written by this kernel.  Tables below 2^28 slots compare whole metadata
+// words (window_masks: about a third of the instructions of the slot by slot
+// walk, which is kept for depths that do not fit the word).
+template <int KB, bool RO = true>
 __device__ __forceinline__ uint64_t get_probe_key(const TableView& t, const RegKey<KB>& key, uint64_t h) {
     const uint64_t mask = t.mask;
+    const uint32_t ksz = KB ? (uint32_t)KB : t.ksz;
+    if (mask < (uint64_t)DIST_MASK) {
+        const uint32_t m32 = (uint32_t)mask, off = (uint32_t)h & 7u;
+        uint32_t wb = (uint32_t)h & ~7u;
+        uint32_t e0 = ST_OCC - (off << 4);
+        uint32_t live = (0xFFu << off) & 0xFFu;
+        for (uint32_t left = (m32 >> 3) + 1;; --left) {  // the home's window comes twice
+            const uint4* fp = reinterpret_cast<const uint4*>(t.flags + (wb & m32));
+            uint4 a, b;
+            if constexpr (RO) a = __ldg(fp), b = __ldg(fp + 1);
+            else a = fp[0], b = fp[1];
+            uint32_t cand, term;
+            window_masks(a, b, e0, cand, term);
+            cand &= live;
+            term &= live;
+            if (term) cand &= (term & (0u - term)) - 1u;
+            while (cand) {  // in walk order
+                const uint64_t slot = (wb + (uint32_t)(__ffs(cand) - 1)) & m32;
+                if (key.eq(t.keys + slot * ksz, ksz)) return slot;
+                cand &= cand - 1;
+            }
+            if (term || left == 0) return NONE64;
+            wb += 8;
+            e0 += 128;
+            live = left == 1 ? (1u << off) - 1u : 0xFFu;
+        }
+    }
     uint64_t wb = h & ~7ull;
     uint64_t hit = NONE64;
     bool done = false;
     while (!done) {
         const uint4* fp = reinterpret_cast<const uint4*>(t.flags + (wb & mask));
-        const uint4 a = __ldg(fp), b = __ldg(fp + 1);
+        const uint4 a = fp[0], b = fp[1];
         const uint32_t f8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         // the window in registers: candidates (stored distance == depth)
         // before the first terminator -- probe past the capacity, EMPTY, or
@@ -82,7 +130,7 @@ __device__ __forceinline__ uint64_t get_probe_key(const TableView& t, const RegK
             const int l = __ffs(cand) - 1;
             cand &= cand - 1;
             const uint64_t slot = (wb + l) & mask;
-            if (key.eq(t.keys + slot * KB, KB)) {
+            if (key.eq(t.keys + slot * ksz, ksz)) {
                 hit = slot;
                 done = true;
                 break;

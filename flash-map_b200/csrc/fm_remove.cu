@@ -554,8 +554,13 @@ template <int KB>
 __device__ __forceinline__ uint32_t rx_take(const TableView& t, const uint8_t* keys, uint32_t j) {
     RegKey<KB> key;
     const uint64_t h = home_of<KB>(t, keys, j, key);
-    uint64_t stop;
-    const uint64_t x = rx_look<KB>(t, key, h, false, &stop);
+    uint64_t x;
+    if (t.mask >= 7) {
+        x = get_probe_key<KB, false>(t, key, h);
+    } else {
+        uint64_t stop;
+        x = rx_look<KB>(t, key, h, false, &stop);
+    }
     return x != NONE64 && st_of(atomicExch(&t.flags[x], ST_TOMB)) == ST_OCC ? 1u : 0u;
 }
 
