@@ -380,8 +380,10 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // (lone ops at once, each group in index order); ops the kernels
             // leave (no EMPTY slot anywhere, groups too large) run in rounds
             // -- or, while no insert has claimed a tombstone, in one pass in
-            // any order
-            const bool any_order = !t->claimed.load() && t->mask < (uint64_t)fm::DIST_MASK;
+            // any order (a table filled to its last slot stays with the rounds
+            // and their bounded passes: it has no EMPTY slot for a probe to end at)
+            const bool any_order = !t->claimed.load() && t->mask < (uint64_t)fm::DIST_MASK &&
+                                   t->len.load() - total < t->cap;
             e = any_order ? fm::launch_rem_take(v, sh, kk, m, t->d_ctl, s)
                           : fm::launch_rem_direct(v, sh, kk, m, t->sc, t->d_ctl, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
@@ -431,7 +433,8 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // index order per component; what the kernels leave (a table with
             // no free slot for some op, components too large for a warp) runs
             // on the component path
-            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, s);
+            const bool clean = t->mask >= 7 && t->mask < (uint64_t)fm::DIST_MASK && !t->tombs.load();
+            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, clean, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;

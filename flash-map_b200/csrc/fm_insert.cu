@@ -27,6 +27,7 @@
 // TAIL_MAX ops are left.  The host reads the control block once per pass.
 // Grid kernels aggregate list appends and counts per block so no address
 // takes more than one atomic per block.
+#include <algorithm>
 #include <climits>
 #include <limits>
 #include <cstdlib>
@@ -73,6 +74,13 @@ __device__ __forceinline__ uint64_t find_free(const TableView& t, const uint8_t*
     return NONE64;
 }
 
+// The OCCUPIED slots of eight metadata words as a mask (EMPTY 0, OCCUPIED with
+// its distance odd, TOMBSTONE 2).
+__device__ __forceinline__ uint32_t occupied8(const uint4& a, const uint4& b) {
+    return (a.x & 1u) | (a.y & 1u) << 1 | (a.z & 1u) << 2 | (a.w & 1u) << 3 | (b.x & 1u) << 4 | (b.y & 1u) << 5 |
+           (b.z & 1u) << 6 | (b.w & 1u) << 7;
+}
+
 // The same from a known home h.  With capacity >= 64: two aligned 8-slot
 // windows in the first round trip (most walks end there), then four per
 // round trip, so a long walk takes fewer trips; smaller tables two windows
@@ -85,10 +93,9 @@ __device__ __forceinline__ uint64_t find_free_from(const TableView& t, uint64_t 
             const uint4* p0 = reinterpret_cast<const uint4*>(t.flags + (wb & mask));
             const uint4* p1 = reinterpret_cast<const uint4*>(t.flags + ((wb + 8) & mask));
             const uint4 a = p0[0], b = p0[1], c = p1[0], d = p1[1];
-            const uint32_t f16[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
-#pragma unroll
-            for (int l = 0; l < 16; l++)
-                if (wb + l >= h && is_free(f16[l])) return (wb + l) & mask;
+            uint32_t free = ~(occupied8(a, b) | occupied8(c, d) << 8) & 0xFFFFu;
+            free &= 0xFFFFu << (uint32_t)(h & 7u);
+            if (free) return (wb + (uint32_t)(__ffs(free) - 1)) & mask;
         }
         for (wb += 16; wb - h <= mask; wb += 32) {
             uint4 x[8];
@@ -98,15 +105,11 @@ __device__ __forceinline__ uint64_t find_free_from(const TableView& t, uint64_t 
                 x[2 * q] = pq[0];
                 x[2 * q + 1] = pq[1];
             }
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const uint32_t f4[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
-#pragma unroll
-                for (int l = 0; l < 4; l++) {
-                    const uint64_t pos = wb + 4 * q + l;
-                    if (pos - h > mask) return NONE64;
-                    if (is_free(f4[l])) return pos & mask;
-                }
+            const uint32_t free = ~(occupied8(x[0], x[1]) | occupied8(x[2], x[3]) << 8 | occupied8(x[4], x[5]) << 16 |
+                                    occupied8(x[6], x[7]) << 24);
+            if (free) {
+                const uint64_t pos = wb + (uint32_t)(__ffs(free) - 1);
+                return pos - h > mask ? NONE64 : pos & mask;
             }
         }
         return NONE64;
@@ -133,6 +136,189 @@ __device__ __forceinline__ uint64_t find_free_from(const TableView& t, uint64_t 
         if (is_free(t.flags[s])) return s;
     }
     return NONE64;
+}
+
+// The evictions of a walk on a table without tombstones, as bits from the
+// 8-slot window that holds the home (DX_BITS slots): see dx_find_warp.
+constexpr uint32_t DX_BITS = 96;
+constexpr uint32_t DX_NOBITS = 0xFFFFFFFFu;  // w[2]: the walk does not fit
+struct DxBits {
+    uint32_t w[3] = {0, 0, DX_NOBITS};
+};
+
+// n metadata words f[0..n) (the one before them in prev) against the words a
+// probing key would have there (e0 + 16 per slot): `eq` has the slots that
+// hold exactly that, the only ones that can hold the key; `less` those of a
+// higher home than the key's or EMPTY, where its probe ends; `turn` those that
+// are not one step of distance after the slot before.
+template <int N>
+__device__ __forceinline__ void order_masks(const uint32_t (&f)[N], uint32_t prev, uint32_t e0, uint32_t& eq,
+                                            uint32_t& less, uint32_t& turn) {
+    eq = 0, less = 0, turn = 0;
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+        if (f[l] == e0 + 16u * l) eq |= 1u << l;
+        if (f[l] < e0 + 16u * l) less |= 1u << l;
+        if (f[l] != (l ? f[l ? l - 1 : 0] : prev) + 16u) turn |= 1u << l;
+    }
+}
+
+// The evictions among a stretch's slots before `valid` ends: the first slot
+// of a higher home, then every change of home.
+__device__ __forceinline__ uint32_t order_evictions(uint32_t less, uint32_t turn, uint32_t valid, bool& started) {
+    uint32_t ev = turn & valid;
+    if (!started) {
+        less &= valid;
+        const uint32_t first = less & (0u - less);
+        started = less != 0;
+        ev = first ? (ev & ~(first - 1u)) | first : 0u;
+    }
+    return ev;
+}
+
+// First free slot at or after h for the lanes of a warp that want it
+// (warp-uniform call): 16 slots on each lane's own, then 32 more; the walks
+// that go on are finished by the whole warp, 256 slots per round trip.  At
+// load 0.8 the longest of 32 walks is often above 100 slots and the longest
+// of a call above 400: on one thread such a walk is a chain of dependent
+// reads, and the pass lasts as long as its longest chain.
+//
+// With `clean` (a table without tombstones; the key is not stored) it also
+// gives the walk's evictions.  The entries of [home, F) are sorted by home
+// there, so these are the first slot of a higher home and then every slot
+// where the home changes: where the metadata word is not the one before it
+// plus one step of distance.  The exec pass then needs no metadata of its
+// own before it moves records.  And the same reads serve the probe for the
+// key, whose slot is returned in hit (NONE64: not stored).
+template <int KB>
+__device__ __forceinline__ uint64_t find_free_warp(const TableView& t, const RegKey<KB>& key, uint64_t h, bool want,
+                                                   bool clean, DxBits& bits, uint64_t& hit) {
+    const uint64_t mask = t.mask;
+    hit = NONE64;
+    if (mask < 511) {
+        if (want && clean) hit = get_probe_key<KB, true>(t, key, h);
+        return want && hit == NONE64 ? find_free_from(t, h) : NONE64;
+    }
+    const uint64_t wb = h & ~7ull;
+    const uint32_t off = (uint32_t)(h & 7u);
+    const uint32_t e0 = ST_OCC - (off << 4);
+    uint64_t F = NONE64;
+    uint32_t end = 0;       // F, as a bit number (may be beyond DX_BITS)
+    uint32_t prev = 0;      // the last word read
+    bool started = false;
+    if (want) {
+        const uint4* p0 = reinterpret_cast<const uint4*>(t.flags + (wb & mask));
+        const uint4* p1 = reinterpret_cast<const uint4*>(t.flags + ((wb + 8) & mask));
+        const uint4 a = p0[0], b = p0[1], c = p1[0], d = p1[1];
+        const uint32_t f[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+        uint32_t free = ~(occupied8(a, b) | occupied8(c, d) << 8) & 0xFFFFu;
+        const uint32_t from = 0xFFFFu << off;
+        free &= from;
+        const uint32_t below = free ? (free & (0u - free)) - 1u : 0xFFFFu;
+        uint32_t eq, less, turn;
+        order_masks<16>(f, 0u, e0, eq, less, turn);
+        unsigned long long cand = eq & from;           // slots that can hold the key, before the probe's end
+        uint32_t stop = less & from & 0xFFFFu;
+        if (stop) cand &= (stop & (0u - stop)) - 1u;
+        bits.w[0] = order_evictions(less, turn, below & from & 0xFFFFu, started);
+        bits.w[1] = 0;
+        if (free) {
+            end = (uint32_t)(__ffs(free) - 1);
+            F = (wb + end) & mask;
+            bits.w[2] = 0;
+        } else {
+            uint4 x[8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint4* pq = reinterpret_cast<const uint4*>(t.flags + ((wb + 16 + 8 * q) & mask));
+                x[2 * q] = pq[0];
+                x[2 * q + 1] = pq[1];
+            }
+            free = ~(occupied8(x[0], x[1]) | occupied8(x[2], x[3]) << 8 | occupied8(x[4], x[5]) << 16 |
+                     occupied8(x[6], x[7]) << 24);
+            const uint32_t g[32] = {x[0].x, x[0].y, x[0].z, x[0].w, x[1].x, x[1].y, x[1].z, x[1].w,
+                                    x[2].x, x[2].y, x[2].z, x[2].w, x[3].x, x[3].y, x[3].z, x[3].w,
+                                    x[4].x, x[4].y, x[4].z, x[4].w, x[5].x, x[5].y, x[5].z, x[5].w,
+                                    x[6].x, x[6].y, x[6].z, x[6].w, x[7].x, x[7].y, x[7].z, x[7].w};
+            order_masks<32>(g, f[15], e0 + 256u, eq, less, turn);
+            if (!stop) {
+                if (less) eq &= (less & (0u - less)) - 1u;
+                cand |= (unsigned long long)eq << 16;
+                stop = less;
+            }
+            const uint32_t ev =
+                order_evictions(less, turn, free ? (free & (0u - free)) - 1u : 0xFFFFFFFFu, started);
+            bits.w[0] |= ev << 16;
+            bits.w[1] = ev >> 16;
+            if (free) {
+                end = 16 + (uint32_t)(__ffs(free) - 1);
+                F = (wb + end) & mask;
+                bits.w[2] = 0;
+            }
+            prev = g[31];
+        }
+        if (clean) {
+            if (!stop) {  // a probe of more than 48 slots
+                hit = get_probe_key<KB, true>(t, key, h);
+            } else {
+                for (; cand; cand &= cand - 1) {  // in walk order
+                    const uint64_t x = (wb + (uint32_t)(__ffsll((long long)cand) - 1)) & mask;
+                    if (key.eq(t.keys + x * KB, KB)) {
+                        hit = x;
+                        break;
+                    }
+                }
+            }
+            if (hit != NONE64) want = false;
+        }
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, want && F == NONE64); todo; todo &= todo - 1) {
+        const int who = __ffs(todo) - 1;
+        const uint64_t hw = __shfl_sync(0xFFFFFFFFu, h, who);
+        const uint32_t pw = __shfl_sync(0xFFFFFFFFu, prev, who);
+        uint64_t got = NONE64;
+        uint32_t lo = 0, hi = 0;  // turn (this lane's slots), less
+        // from the 48 slots passed on (aligned down to 8), round the table
+        for (uint64_t b = (hw & ~7ull) + 48; b - hw <= mask; b += 256) {
+            const uint4 f = *reinterpret_cast<const uint4*>(t.flags + ((b + 4 * lane) & mask));
+            const uint4 g = *reinterpret_cast<const uint4*>(t.flags + ((b + 128 + 4 * lane) & mask));
+            const uint32_t ff = ~((f.x & 1u) | (f.y & 1u) << 1 | (f.z & 1u) << 2 | (f.w & 1u) << 3) & 15u;
+            const uint32_t fg = ~((g.x & 1u) | (g.y & 1u) << 1 | (g.z & 1u) << 2 | (g.w & 1u) << 3) & 15u;
+            const uint32_t mf = __ballot_sync(0xFFFFFFFFu, ff != 0), mg = __ballot_sync(0xFFFFFFFFu, fg != 0);
+            if (clean && b - hw < 64) {  // the slots that still have bits: 48 of them, 12 lanes
+                const uint32_t f4[4] = {f.x, f.y, f.z, f.w};
+                const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, f.w, 1);
+                const uint32_t ew = ST_OCC - ((uint32_t)(hw & 7u) << 4) + 16u * (48u + 4u * lane);
+                uint32_t eq;
+                order_masks<4>(f4, lane ? before : pw, ew, eq, hi, lo);
+            }
+            if (mf | mg) {
+                const int l = __ffs(mf ? mf : mg) - 1;
+                const uint32_t bt = __shfl_sync(0xFFFFFFFFu, mf ? ff : fg, l);
+                got = b + (mf ? 0 : 128) + 4 * l + (uint32_t)(__ffs(bt) - 1);
+                if (got - hw > mask) got = NONE64;
+                break;
+            }
+        }
+        if (clean) {
+            // slots 48..79 and 80..95 of the walk
+            const uint32_t t0 = __reduce_or_sync(0xFFFFFFFFu, lane < 8 ? lo << (4 * lane) : 0u);
+            const uint32_t t1 = __reduce_or_sync(0xFFFFFFFFu, lane >= 8 && lane < 12 ? lo << (4 * (lane - 8)) : 0u);
+            const uint32_t l0 = __reduce_or_sync(0xFFFFFFFFu, lane < 8 ? hi << (4 * lane) : 0u);
+            const uint32_t l1 = __reduce_or_sync(0xFFFFFFFFu, lane >= 8 && lane < 12 ? hi << (4 * (lane - 8)) : 0u);
+            if ((int)lane == who && got != NONE64 && got - wb < DX_BITS) {
+                const uint32_t n = (uint32_t)(got - wb) - 48;  // slots before F there
+                const uint32_t v0 = n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u, v1 = n > 32 ? (1u << (n - 32)) - 1u : 0u;
+                const uint32_t ev0 = order_evictions(l0, t0, v0, started);
+                const uint32_t ev1 = order_evictions(l1, t1, v1, started);
+                bits.w[1] |= ev0 << 16;
+                bits.w[2] = ev0 >> 16 | ev1 << 16;
+            }
+        }
+        if ((int)lane == who && got != NONE64) F = got & mask;
+    }
+    return F;
 }
 
 __device__ __forceinline__ void register_op(const TableView& t, uint32_t j, uint64_t F, uint64_t* op_slot) {
@@ -1999,10 +2185,12 @@ __global__ void __launch_bounds__(RBLOCK) k_cmp_clean(TableView t, OpScratch sc)
 //         the records moved two per round trip; a walk too long for one
 //         thread, and the leader of an unmarked F with c >= 2, go to the warp
 //         pass's list; the other ops wait for their component.
-//   warp  (a warp per list entry)  a long lone op runs as a tile walk; a
-//         component gathers its ops from the lists of its free slots (the
-//         flow walk again), sorts them by index and runs them one after
-//         another as tile walks.
+//   cf    (a warp per list entry; tables without tombstones)  a component
+//         gathers its ops from the lists of its free slots (the flow walk
+//         again), sorts them by index and does what they do at once; a long
+//         lone op likewise.
+//   warp  (a warp per list entry; other tables, and what cf leaves)  a long
+//         lone op runs as a tile walk; a component's ops one after another.
 // Components touch disjoint slots, so all of this runs at once.  A call that
 // finds an op with no free slot or a flow round the whole table leaves every
 // op to the component path (Ctl::serial[0]); a component with more ops than a
@@ -2012,17 +2200,26 @@ constexpr uint32_t DX_ABS = 0x80000000u;   // seg_cnt: the free slot is in an ea
 constexpr uint32_t DX_CNT = 0x7FFFFFFFu;
 constexpr uint32_t DX_ROOT = 0x80000000u;  // warp-pass list entry: a component's leader
 constexpr uint64_t DX_UPDATE = 1ull << 63; // op_slot: an update of that slot (tables without tombstones)
+// op_flag on tables without tombstones: 0 not the first op at its free slot,
+// 1 alone there, DX_CROWDED the first of several, DX_TAKEN alone there but in
+// an earlier slot's component (so the exec pass need not read seg_cnt).
+constexpr uint8_t DX_CROWDED = 2, DX_TAKEN = 3;
 #ifndef FM_DX_LCH
-#define FM_DX_LCH 8
+#define FM_DX_LCH 24
 #endif
 #ifndef FM_DX_LTRIPS
-#define FM_DX_LTRIPS 4
+#define FM_DX_LTRIPS 8
 #endif
 constexpr int DX_LCH = FM_DX_LCH;          // evictions of a walk on the thread path
 constexpr int DX_LCMP = 6;                 // possible updates of a walk on the thread path
 constexpr int DX_LTRIPS = FM_DX_LTRIPS;    // 16-slot metadata reads of a walk on the thread path
+#ifndef FM_DX_BLOCKS
+#define FM_DX_BLOCKS 2
+#endif
+constexpr int DX_BLOCKS = FM_DX_BLOCKS;    // resident exec blocks per SM
 constexpr int DX_GATHER = 64;              // ops of a component the warp pass runs itself
 constexpr int DX_THREADS = 256;            // threads of an exec block
+static_assert(16 * DX_LTRIPS < 256 && DX_LCH < 256, "walk offsets and moves in bytes");
 
 // Programmatic dependent launch between the direct kernels (compile-time
 // setting FM_DX_PDL, default on): each kernel lets the next one launch as
@@ -2056,6 +2253,28 @@ __device__ __forceinline__ bool dx_clean(const TableView& t, const Ctl* ctl) {
 // `budget` slots (less the slots looked at); NONE64 when none lies within it.
 __device__ __forceinline__ uint64_t dx_next_free(const TableView& t, uint64_t a, uint64_t& budget) {
     const uint64_t mask = t.mask;
+    if (mask >= 63) {
+        // 32 slots per round trip (the last trip may look past the budget)
+        uint32_t seen = (uint32_t)(a & 7u);
+        for (uint64_t wb = a & ~7ull; budget > 0; wb += 32, seen = 0) {
+            uint4 x[8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint4* pq = reinterpret_cast<const uint4*>(t.flags + ((wb + 8 * q) & mask));
+                x[2 * q] = pq[0];
+                x[2 * q + 1] = pq[1];
+            }
+            uint32_t free = ~(occupied8(x[0], x[1]) | occupied8(x[2], x[3]) << 8 | occupied8(x[4], x[5]) << 16 |
+                              occupied8(x[6], x[7]) << 24);
+            free &= 0xFFFFFFFFu << seen;
+            const uint32_t n = free ? (uint32_t)__ffs(free) - seen : 32u - seen;  // slots looked at
+            if (n > budget) break;
+            budget -= n;
+            if (free) return wb + (uint32_t)(__ffs(free) - 1);
+        }
+        budget = 0;
+        return NONE64;
+    }
     if (mask >= 7) {
         for (uint64_t wb = a & ~7ull; budget > 0; wb += 8) {
             const uint4* fp = reinterpret_cast<const uint4*>(t.flags + (wb & mask));
@@ -2086,23 +2305,28 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_find(TableView t, const uint8_t* 
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
     const bool clean = dx_clean(t, ctl);
     bool no_free = false;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x) {
+    const uint32_t iters = grid_iters(n0);
+    for (uint32_t it = 0; it < iters; it++) {  // warp-uniform trip count
+        const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x + it * gridDim.x * blockDim.x;
+        uint64_t h = 0, x;
         RegKey<KB> key;
-        key.load(keys + (uint64_t)j * KB, KB);
-        const uint64_t h = key.hash(KB, t.hash_mode) & t.mask;
-        if (clean) {
-            const uint64_t x = get_probe_key<KB>(t, key, h);
-            if (x != NONE64) {  // an update of slot x: the last op on it wins
-                sc.op_slot[j] = x | DX_UPDATE;
-                sc.op_word[j] = IDLE;
-                sc.op_flag[j] = 0;
-                atomicMin(&t.seg_min[x], upd_code(j));
-                continue;
-            }
+        if (j < n0) {
+            key.load(keys + (uint64_t)j * KB, KB);
+            h = key.hash(KB, t.hash_mode) & t.mask;
         }
-        const uint64_t F = find_free_from(t, h);
+        DxBits bits;
+        const uint64_t F = find_free_warp<KB>(t, key, h, j < n0, clean, bits, x);
+        if (j >= n0) continue;
+        if (x != NONE64) {  // an update of slot x: the last op on it wins
+            sc.op_slot[j] = x | DX_UPDATE;
+            sc.op_word[j] = IDLE;
+            sc.op_flag[j] = 0;
+            atomicMin(&t.seg_min[x], upd_code(j));
+            continue;
+        }
         sc.op_slot[j] = F;
-        sc.op_pt[(uint64_t)j * PT_MAX] = (uint32_t)h;  // the exec pass starts from it
+        // the exec pass starts from these
+        reinterpret_cast<uint4*>(sc.op_pt)[j] = make_uint4((uint32_t)h, bits.w[0], bits.w[1], bits.w[2]);
         uint8_t lead = 0;
         uint32_t next = IDLE;
         if (F == NONE64) {
@@ -2146,6 +2370,7 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, const uint8_t* 
         const uint64_t F = sc.op_slot[j];
         const uint32_t c = t.seg_cnt[F] & DX_CNT;
         if (c < 2) continue;
+        if (clean) sc.op_flag[j] = DX_CROWDED;
         uint64_t flow = c - 1, a = F + 1, budget = t.mask;  // back at F: the flow wraps the table
         for (;;) {
             const uint64_t at = dx_next_free(t, a, budget);
@@ -2162,6 +2387,7 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, const uint8_t* 
                     break;
                 }
                 if (!(w2 & DX_ABS)) atomicOr(&t.seg_cnt[F2], DX_ABS);
+                if (clean && c2 == 1) sc.op_flag[t.seg_min[F2]] = DX_TAKEN;
             }
             flow = flow + c2 - 1;
             if (flow == 0) break;
@@ -2171,12 +2397,13 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, const uint8_t* 
 }
 
 // The thread path's per-thread lists (shared memory, one column per thread):
-// eviction slots and depths, possible-update slots and the evictions before
-// each; and per warp the moves of its ops (lane << 8 | move).
+// eviction slots (from the op's home) and depths, possible-update slots and
+// the evictions before each; and per warp the moves of its ops (lane << 8 |
+// move).  A walk spans fewer than 256 slots, so bytes hold them.
 struct DxLaneSmem {
-    uint32_t pos[DX_LCH][DX_THREADS];
-    uint32_t dep[DX_LCH][DX_THREADS];
-    uint32_t cpos[DX_LCMP][DX_THREADS];
+    uint8_t pos[DX_LCH][DX_THREADS];
+    uint8_t dep[DX_LCH][DX_THREADS];
+    uint8_t cpos[DX_LCMP][DX_THREADS];
     uint8_t cst[DX_LCMP][DX_THREADS];
     uint16_t list[DX_THREADS / 32][32 * (DX_LCH + 1)];
 };
@@ -2210,70 +2437,76 @@ struct DxPlan {
 // resident is carried on: H = r), one with r == H is a possible update, and F
 // takes the last carried entry.  The possible updates are compared on the
 // keys' first 8 bytes, all in one round trip, and in full only where those
-// agree (the first equal key in walk order ends the walk in place); with
-// `fresh` (the key is not stored, on a table where no key is stored twice)
-// there is nothing to compare.  Reads only.  -1 when the walk needs more than
+// agree (the first equal key in walk order ends the walk in place).  Reads only.  -1 when the walk needs more than
 // DX_LTRIPS metadata reads, DX_LCH evictions or DX_LCMP possible updates, or
 // when the metadata does not show F as the first free slot.  Needs capacity
 // >= 8 and below 2^28 slots.
 template <int KB>
 __device__ __forceinline__ DxPlan dx_plan(const TableView& t, const RegKey<KB>& key, uint64_t h, uint64_t F,
-                                          const DxWin& w0, bool fresh, DxLaneSmem& sl) {
+                                          const DxWin& w0, DxLaneSmem& sl) {
     DxPlan p;
     p.kind = -1;
-    const uint64_t mask = t.mask;
+    const uint32_t m32 = (uint32_t)t.mask, h32 = (uint32_t)h;
     const uint32_t me = threadIdx.x;
-    const uint64_t e = h + ((F - h) & mask);  // F, unwrapped
-    const uint64_t wb = h & ~7ull;
-    if (e - wb >= 16ull * DX_LTRIPS) return p;
+    // positions from the home on; the carried entry's home H likewise
+    const uint32_t e = ((uint32_t)F - h32) & m32;
+    const uint32_t off = h32 & 7u;
+    if (e + off >= 16u * DX_LTRIPS) return p;
     uint32_t k = 0, nc = 0;
-    long long H = (long long)h;
+    int H = 0;
     bool end_tomb = false;
-    for (uint64_t w = wb; w <= e; w += 16) {
+    for (int w = -(int)off; w <= (int)e; w += 16) {
         DxWin win = w0;
-        if (w != wb) win.load(t, w);
+        if (w > 0) win.load(t, (uint64_t)(h32 + (uint32_t)w));
         const uint4 fa = win.a, fb = win.b, fc = win.c, fd = win.d;
         const uint32_t f16[16] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w,
                                   fc.x, fc.y, fc.z, fc.w, fd.x, fd.y, fd.z, fd.w};
+        // the slots of [home, F] in this window: OCCUPIED up to F, F not
+        const uint32_t lo = w < 0 ? off : 0u;
+        const uint32_t hi = (int)e - w < 15 ? (uint32_t)((int)e - w) : 16u;  // F's place, 16: further on
+        const uint32_t want = ((1u << hi) - 1u) & (0xFFFFu << lo);
+        const uint32_t occ = occupied8(fa, fb) | occupied8(fc, fd) << 8;
+        if ((occ & want) != want) return p;  // a free slot before F: not what the find pass saw
+        if (hi < 16u) {
+            if (occ >> hi & 1u) return p;
+#pragma unroll
+            for (int l = 0; l < 16; l++)
+                if (l == (int)hi) end_tomb = f16[l] == ST_TOMB;
+        }
 #pragma unroll
         for (int l = 0; l < 16; l++) {
-            const uint64_t pos = w + l;
-            if (pos < h || pos > e) continue;
-            if (pos == e) {
-                if (!is_free(f16[l])) return p;  // not the free slot the find pass saw
-                end_tomb = st_of(f16[l]) == ST_TOMB;
-                continue;
-            }
-            if (st_of(f16[l]) != ST_OCC) return p;  // a free slot before F: likewise
-            const long long r = (long long)pos - (long long)dist_of(f16[l]);
+            if (!(want >> l & 1u)) continue;
+            const int q = w + l;
+            const int r = q - (int)(f16[l] >> 4);
             if (r > H) {
                 if (k == (uint32_t)DX_LCH) return p;
-                sl.pos[k][me] = (uint32_t)(pos & mask);
-                sl.dep[k][me] = (uint32_t)((long long)pos - H);
+                sl.pos[k][me] = (uint8_t)q;
+                sl.dep[k][me] = (uint8_t)(q - H);
                 ++k;
                 H = r;
-            } else if (r == H && !fresh) {
+            } else if (r == H) {
                 if (nc == (uint32_t)DX_LCMP) return p;
-                sl.cpos[nc][me] = (uint32_t)(pos & mask);
+                sl.cpos[nc][me] = (uint8_t)q;
                 sl.cst[nc][me] = (uint8_t)k;
                 ++nc;
             }
         }
     }
     p.kind = 1;
-    p.end = (uint32_t)(e & mask);
-    p.dep = (uint32_t)((long long)e - H);
+    p.end = (uint32_t)F;
+    p.dep = e - (uint32_t)H;
     p.k = k;
     p.tomb = end_tomb;
+    auto slot = [&](uint32_t q) { return (uint64_t)((h32 + q) & m32); };
     if (nc) {
         uint2 rp[DX_LCMP], cp[DX_LCMP];
         const uint2 kp = make_uint2(key.w[0], KB >= 8 ? key.w[1] : 0u);
 #pragma unroll
         for (int c = 0; c < DX_LCMP; c++) {
             if (c < (int)nc) {
-                rp[c] = *reinterpret_cast<const uint2*>(t.keys + (uint64_t)sl.cpos[c][me] * KB);
+                rp[c] = *reinterpret_cast<const uint2*>(t.keys + slot(sl.cpos[c][me]) * KB);
                 const uint32_t st = sl.cst[c][me];
-                cp[c] = st ? *reinterpret_cast<const uint2*>(t.keys + (uint64_t)sl.pos[st - 1][me] * KB) : kp;
+                cp[c] = st ? *reinterpret_cast<const uint2*>(t.keys + slot(sl.pos[st - 1][me]) * KB) : kp;
             }
         }
         for (int c = 0; c < (int)nc; c++) {
@@ -2283,12 +2516,12 @@ __device__ __forceinline__ DxPlan dx_plan(const TableView& t, const RegKey<KB>& 
                 if (q == c) agree = rp[q].x == cp[q].x && rp[q].y == cp[q].y;
             if (!agree) continue;
             const uint32_t st = sl.cst[c][me];
-            const uint32_t cs = sl.cpos[c][me];
+            const uint64_t cs = slot(sl.cpos[c][me]);
             RegKey<KB> ck;
-            if (st) ck.load_table(t.keys + (uint64_t)sl.pos[st - 1][me] * KB, KB);
+            if (st) ck.load_table(t.keys + slot(sl.pos[st - 1][me]) * KB, KB);
             else ck = key;
-            if (ck.eq(t.keys + (uint64_t)cs * KB, KB)) {
-                p.kind = 2, p.end = cs, p.k = st, p.tomb = false;
+            if (ck.eq(t.keys + cs * KB, KB)) {
+                p.kind = 2, p.end = (uint32_t)cs, p.k = st, p.tomb = false;
                 break;
             }
         }
@@ -2296,23 +2529,65 @@ __device__ __forceinline__ DxPlan dx_plan(const TableView& t, const RegKey<KB>& 
     return p;
 }
 
+// Up to BM records moved by a warp: record e < nb (lane e's ks, vs: the slots
+// holding the key and the value, MOVE_NEW | op for an op's own) to slot dst of
+// lane e; a key with keep set stays.  All are loaded before any is stored.
+// Consecutive lanes take consecutive 16-byte pieces (8 for records not of
+// whole 16s), so an instruction covers whole records instead of one piece of
+// 32 scattered ones: with a record per lane the account shape's moves were
+// bound by 20 scattered pieces per record in the L1.  The loads are not
+// conditional (lanes from nb on name a slot of the table as their source), so
+// they are all in flight together; the step lasts one read and one write.
+constexpr uint32_t MOVE_NEW = 0x80000000u;
+template <int KB, int VB, int BM>
+__device__ __forceinline__ void warp_move(const TableView& t, const uint8_t* __restrict__ keys,
+                                          const uint8_t* __restrict__ vals, uint32_t nb, uint32_t ks, uint32_t vs,
+                                          uint32_t dst, bool keep = false) {
+    using CO = ChunkOf<KB, VB>;
+    using Ch = typename CO::type;
+    constexpr int NK = CO::NK, NV = CO::NV;
+    static_assert(32 % NK == 0 && 32 % NV == 0, "whole records per row");
+    constexpr int RK = BM * NK / 32 > 0 ? BM * NK / 32 : 1, RV = BM * NV / 32 > 0 ? BM * NV / 32 : 1;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t kd = keep ? 0xFFFFFFFFu : dst;  // slots are below 2^28
+    Ch kb[RK], vb[RV];
+#pragma unroll
+    for (int u = 0; u < RK; u++) {
+        const uint32_t s = __shfl_sync(0xFFFFFFFFu, ks, (u * (32 / NK) + lane / NK) & 31u);
+        kb[u] = reinterpret_cast<const Ch*>((s & MOVE_NEW ? keys : t.keys) + (uint64_t)(s & ~MOVE_NEW) * KB)[lane % NK];
+    }
+#pragma unroll
+    for (int u = 0; u < RV; u++) {
+        const uint32_t s = __shfl_sync(0xFFFFFFFFu, vs, (u * (32 / NV) + lane / NV) & 31u);
+        vb[u] = reinterpret_cast<const Ch*>((s & MOVE_NEW ? vals : t.vals) + (uint64_t)(s & ~MOVE_NEW) * VB)[lane % NV];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < RK; u++) {
+        const uint32_t e = u * (32 / NK) + lane / NK;
+        const uint32_t d = __shfl_sync(0xFFFFFFFFu, kd, e & 31u);
+        if (e < nb && d != 0xFFFFFFFFu) reinterpret_cast<Ch*>(t.keys + (uint64_t)d * KB)[lane % NK] = kb[u];
+    }
+#pragma unroll
+    for (int u = 0; u < RV; u++) {
+        const uint32_t e = u * (32 / NV) + lane / NV;
+        const uint32_t d = __shfl_sync(0xFFFFFFFFu, dst, e & 31u);
+        if (e < nb) reinterpret_cast<Ch*>(t.vals + (uint64_t)d * VB)[lane % NV] = vb[u];
+    }
+}
+
 // The moves that the plans of a warp's 32 ops ask for (op j of each lane):
 // move m of an op writes P_m (the m-th eviction slot; the end slot for m = k)
 // from P_(m-1) (the new entry for m = 0).  The warp lists them, each op's
-// highest first, and runs 32 at a time together, one 16-byte piece (8 for
-// records not of whole 16s) per lane and step, so that an instruction covers
-// whole records instead of one piece of 32 scattered ones.  A batch loads all
-// its records before it stores any, and later batches read only slots below
-// the ones stored, so each slot is read before it is written.  Ops of
+// highest first, and runs 32 at a time together (warp_move).  A batch loads
+// all its records before it stores any, and later batches read only slots
+// below the ones stored, so each slot is read before it is written.  Ops of
 // different lanes touch disjoint slots.  Warp-uniform call.
 template <int KB, int VB>
 __device__ __forceinline__ void dx_moves(const TableView& t, const uint8_t* __restrict__ keys,
-                                         const uint8_t* __restrict__ vals, uint32_t j, const DxPlan& p,
+                                         const uint8_t* __restrict__ vals, uint32_t j, uint32_t h, const DxPlan& p,
                                          DxLaneSmem& sl, ExecAcc& acc) {
-    using CO = ChunkOf<KB, VB>;
-    using Ch = typename CO::type;
-    constexpr int CK = CO::CK, NK = CO::NK, NP = CO::NC;
-    constexpr uint32_t NEW = 0x80000000u;      // the source is the new entry of an op
+    constexpr uint32_t BM = 32;                   // moves of a batch
     constexpr uint32_t VALUE_ONLY = 0xFFFFFFFFu;  // depth of an update in place
     const uint32_t lane = threadIdx.x & 31u, wb = threadIdx.x & ~31u;
     uint16_t* list = sl.list[threadIdx.x >> 5];
@@ -2328,42 +2603,22 @@ __device__ __forceinline__ void dx_moves(const TableView& t, const uint8_t* __re
     __syncwarp();
     const uint32_t dep_end = p.kind == 2 ? VALUE_ONLY : p.dep;
     uint32_t md = 0;
-    for (uint32_t b = 0; b < total; b += 32) {
-        const uint32_t nb = min(32u, total - b);
+    for (uint32_t b = 0; b < total; b += BM) {
+        const uint32_t nb = min(BM, total - b);
         const uint32_t code = lane < nb ? list[b + lane] : lane << 8;
         const uint32_t ow = code >> 8, m = code & 255u;
         const uint32_t ok = __shfl_sync(0xFFFFFFFFu, p.k, ow);
         const uint32_t oe = __shfl_sync(0xFFFFFFFFu, p.end, ow);
         const uint32_t od = __shfl_sync(0xFFFFFFFFu, dep_end, ow);
         const uint32_t oj = __shfl_sync(0xFFFFFFFFu, j, ow);
+        const uint32_t oh = __shfl_sync(0xFFFFFFFFu, h, ow);
         uint32_t src = 0, dst = 0, dep = VALUE_ONLY;
         if (lane < nb) {
-            src = m ? sl.pos[m - 1][wb + ow] : oj | NEW;
-            dst = m < ok ? sl.pos[m][wb + ow] : oe;
+            src = m ? (oh + sl.pos[m - 1][wb + ow]) & (uint32_t)t.mask : oj | MOVE_NEW;
+            dst = m < ok ? (oh + sl.pos[m][wb + ow]) & (uint32_t)t.mask : oe;
             dep = m < ok ? sl.dep[m][wb + ow] : od;
         }
-        Ch buf[NP];
-#pragma unroll
-        for (int u = 0; u < NP; u++) {
-            const uint32_t g = lane + 32u * u, e = g / NP, c = g % NP;
-            const uint32_t s = __shfl_sync(0xFFFFFFFFu, src, e);
-            const uint32_t d = __shfl_sync(0xFFFFFFFFu, dep, e);
-            if (e >= nb || (d == VALUE_ONLY && c < (uint32_t)NK)) continue;
-            const uint64_t si = s & ~NEW;
-            const uint8_t* from = c < (uint32_t)NK ? (s & NEW ? keys : t.keys) + si * KB + c * CK
-                                                   : (s & NEW ? vals : t.vals) + si * VB + (c - NK) * CK;
-            buf[u] = *reinterpret_cast<const Ch*>(from);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < NP; u++) {
-            const uint32_t g = lane + 32u * u, e = g / NP, c = g % NP;
-            const uint64_t ds = __shfl_sync(0xFFFFFFFFu, dst, e);
-            const uint32_t d = __shfl_sync(0xFFFFFFFFu, dep, e);
-            if (e >= nb || (d == VALUE_ONLY && c < (uint32_t)NK)) continue;
-            uint8_t* to = c < (uint32_t)NK ? t.keys + ds * KB + c * CK : t.vals + ds * VB + (c - NK) * CK;
-            *reinterpret_cast<Ch*>(to) = buf[u];
-        }
+        warp_move<KB, VB, BM>(t, keys, vals, nb, src, src, dst, dep == VALUE_ONLY);
         if (dep != VALUE_ONLY) {
             t.flags[dst] = mk_flag(ST_OCC, dep);
             md = max(md, dep);
@@ -2377,10 +2632,127 @@ __device__ __forceinline__ void dx_moves(const TableView& t, const uint8_t* __re
     acc.maxd = max(acc.maxd, md);
 }
 
+// The exec pass on tables without tombstones: an op alone at its free slot,
+// with the evictions that the find pass gave as bits.  The word written at
+// each destination is the one before it plus one step of distance (the entry
+// carried there is of the home of the slots just passed), but for the op's
+// own entry.  The warp lists its ops' destinations, each op's highest first,
+// and moves 32 records at a time (warp_move; a batch reads the slots below
+// the ones it and earlier batches write).  Components and walks that do not
+// fit the bits go to the component pass's list.  Bound by the latency of the
+// moves' reads: few registers, so that the ops of a 100K call are all
+// resident at once.
+constexpr int DC_THREADS = 128;
+#ifndef FM_DC_BATCH
+#define FM_DC_BATCH 16
+#endif
+#ifndef FM_DC_BLOCKS
+#define FM_DC_BLOCKS 6
+#endif
+template <int KB, int VB>
+__global__ void __launch_bounds__(DC_THREADS, FM_DC_BLOCKS) k_dx_exec_clean(TableView t, const uint8_t* __restrict__ keys,
+                                                                 const uint8_t* __restrict__ vals, uint32_t n0_arg,
+                                                                 uint32_t opw, OpScratch sc, Ctl* ctl) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu, OWN = 0x2000u;  // list: lane << 8 | bit, OWN: the op's own entry
+    constexpr uint32_t BM = FM_DC_BATCH;
+    __shared__ uint16_t s_list[DC_THREADS / 32][32 * (DX_LCH + 1) + 1];
+    __shared__ uint32_t s_tmp[DC_THREADS / 32];
+    dx_wait_prev();
+    dx_let_next();
+    if (!dx_clean(t, ctl)) return;  // block-uniform
+    const uint32_t n0 = cmp_n0(n0_arg, ctl);
+    const bool to_pend = n0_arg == CMP_N0_CTL;  // as k_dx_exec
+    const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;
+    const uint32_t lane = threadIdx.x & 31u, m32 = (uint32_t)t.mask;
+    uint16_t* list = s_list[threadIdx.x >> 5];
+    uint32_t claimed = 0, md = 0;
+    // opw ops per warp: in a small call fewer, so that the moves of its ops,
+    // one batch after another, spread over the chip
+    for (uint32_t j0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * opw; j0 < n0;
+         j0 += (gridDim.x * blockDim.x >> 5) * opw) {
+        const uint32_t j = j0 + lane;
+        const bool mine = lane < opw && j < n0;
+        uint64_t F = NONE64;
+        uint32_t fl = 0;
+        uint4 w = make_uint4(0, 0, 0, 0);
+        if (mine) {
+            F = sc.op_slot[j];
+            fl = sc.op_flag[j];
+            w = reinterpret_cast<const uint4*>(sc.op_pt)[j];
+        }
+        if (serial) {  // registrations back to idle; the component path runs every op
+            if (mine && to_pend) sc.pend[1][atomicAdd(&ctl->npend[1], 1u)] = j;
+            if (F <= t.mask) {
+                t.seg_min[F] = IDLE;
+                t.seg_cnt[F] = 0;
+                sc.op_word[j] = IDLE;
+            }
+            continue;
+        }
+        if (F > t.mask) fl = 0;  // an update, done
+        bool defer = false;
+        uint32_t cnt = 0;
+        if (fl == 1) {
+            cnt = (uint32_t)(__popc(w.y) + __popc(w.z) + __popc(w.w)) + 1u;
+            if (w.w == DX_NOBITS || cnt > (uint32_t)DX_LCH + 1u) defer = true, cnt = 0;
+            t.seg_min[F] = IDLE;
+            t.seg_cnt[F] = 0;
+            sc.op_word[j] = IDLE;
+        } else if (fl == DX_CROWDED) {
+            defer = !(t.seg_cnt[F] & DX_ABS);
+        }
+        append(sc.long_list, &ctl->nlong[0], fl == 1 ? j : j | DX_ROOT, defer);
+        __syncwarp();
+        uint32_t inc = cnt;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(FULL, inc, d);
+            if ((int)lane >= d) inc += o;
+        }
+        const uint32_t total = __shfl_sync(FULL, inc, 31);
+        if (cnt) {  // destinations, highest first: F, then the evictions
+            uint16_t* out = list + (inc - cnt);
+            *out++ = (uint16_t)(lane << 8 | (((uint32_t)F - (w.x & ~7u)) & m32));
+            const uint32_t b3[3] = {w.y, w.z, w.w};
+#pragma unroll
+            for (int q = 2; q >= 0; q--) {
+                for (uint32_t b = b3[q]; b;) {
+                    const int x = 31 - __clz(b);
+                    *out++ = (uint16_t)(lane << 8 | (32 * q + x));
+                    b ^= 1u << x;
+                }
+            }
+            out[-1] |= (uint16_t)OWN;  // the lowest takes the op's entry
+            ++claimed;
+        }
+        __syncwarp();
+        for (uint32_t b = 0; b < total; b += BM) {
+            const uint32_t nb = min(BM, total - b);
+            const uint32_t at = b + min(lane, nb - 1u);  // lanes from nb on: as the last one, not stored
+            const uint32_t code = list[at], below = list[at + 1];
+            const uint32_t ow = code >> 8 & 31u;
+            const uint32_t oh = __shfl_sync(FULL, w.x, ow);
+            const uint32_t oj = __shfl_sync(FULL, j, ow);
+            const uint32_t hb = oh & ~7u;
+            const uint32_t dst = (hb + (code & 255u)) & m32;
+            const uint32_t before = t.flags[(dst - 1u) & m32];
+            // the op's own entry, or the one from the next destination below
+            const uint32_t src = code & OWN ? oj | MOVE_NEW : (hb + (below & 255u)) & m32;
+            warp_move<KB, VB, BM>(t, keys, vals, nb, src, src, dst);
+            const uint32_t flag = code & OWN ? mk_flag(ST_OCC, (code & 255u) - (oh & 7u)) : before + 16u;
+            if (lane < nb) t.flags[dst] = flag;
+            md = max(md, flag >> 4);
+            __syncwarp();
+        }
+    }
+    block_add_count(ctl, claimed, s_tmp);
+    publish_rare(ctl, md, false, false);
+}
+
 // The exec pass: one thread per op (uniform trip count per warp, for the
 // warp-aggregated appends).
 template <int KB, int VB>
-__global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const uint8_t* __restrict__ keys,
+__global__ void __launch_bounds__(DX_THREADS, DX_BLOCKS) k_dx_exec(TableView t, const uint8_t* __restrict__ keys,
                                                            const uint8_t* __restrict__ vals, uint32_t n0_arg,
                                                            OpScratch sc, Ctl* ctl) {
     __shared__ DxLaneSmem s_lane;
@@ -2394,29 +2766,30 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
     const bool to_pend = n0_arg == CMP_N0_CTL;
     const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;
     const bool lanes_ok = t.mask >= 7 && t.mask < (uint64_t)DIST_MASK;
-    const bool fresh = dx_clean(t, ctl);  // updates are done: every op left has a key that is not stored
+    if (dx_clean(t, ctl)) return;  // block-uniform: k_dx_exec_clean
     ExecAcc a;
-    // ops taken 32 at a time per warp from a counter (Ctl::exec_next, zero at
-    // the start of the call): the grid is the resident blocks, and a warp that
-    // drew long walks does not hold up a static share of the ops
-    for (;;) {
-        uint32_t j0 = 0;
-        if ((threadIdx.x & 31u) == 0) j0 = atomicAdd(&ctl->exec_next, 32u);
-        j0 = __shfl_sync(0xFFFFFFFFu, j0, 0);
+    // ops taken 32 at a time per warp, after the first from a counter
+    // (Ctl::exec_next, zero at the start of the call): the grid is the resident
+    // blocks, and a warp that drew long walks does not hold up a static share
+    uint32_t j0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;  // a warp's first ops are its own
+    const uint32_t behind = gridDim.x * blockDim.x;
+    for (;; j0 = __shfl_sync(0xFFFFFFFFu, j0, 0)) {
         if (j0 >= n0) break;
         const uint32_t j = j0 + (threadIdx.x & 31u);
         uint32_t item = 0;
         bool defer = false;
         DxPlan p;
+        uint32_t h32 = 0;
         if (j < n0 && serial && to_pend) sc.pend[1][atomicAdd(&ctl->npend[1], 1u)] = j;
         if (j < n0) {
             // independent loads together: free slot, home, key; then the
             // registration count with the first metadata window
             const uint64_t F = sc.op_slot[j];
             const uint64_t h = sc.op_pt[(uint64_t)j * PT_MAX];
+            h32 = (uint32_t)h;
             RegKey<KB> key;
-            if (!fresh) key.load(keys + (uint64_t)j * KB, KB);
-            if (F <= t.mask) {  // not an update, and a free slot
+            key.load(keys + (uint64_t)j * KB, KB);
+            if (F <= t.mask) {
                 DxWin w0;
                 if (lanes_ok && !serial) w0.load(t, h & ~7ull);
                 const uint32_t w = t.seg_cnt[F];
@@ -2426,7 +2799,7 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
                     sc.op_word[j] = IDLE;
                 } else if (w == 1u) {  // alone at F, and F in no other op's component
                     p.kind = -1;
-                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, fresh, s_lane);
+                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, s_lane);
                     if (p.kind < 0) defer = true, item = j;
                     t.seg_min[F] = IDLE;
                     t.seg_cnt[F] = 0;
@@ -2438,7 +2811,8 @@ __global__ void __launch_bounds__(DX_THREADS, 2) k_dx_exec(TableView t, const ui
         }
         append(sc.long_list, &ctl->nlong[0], item, defer);
         __syncwarp();
-        dx_moves<KB, VB>(t, keys, vals, j, p, s_lane, a);
+        dx_moves<KB, VB>(t, keys, vals, j, h32, p, s_lane, a);
+        if ((threadIdx.x & 31u) == 0) j0 = behind + atomicAdd(&ctl->exec_next, 32u);
     }
     block_add_count(ctl, a.claimed, s_tmp);
     publish_rare(ctl, a.maxd, a.tomb, a.limit);
@@ -2458,56 +2832,55 @@ __device__ __forceinline__ void dx_run_tile(const TableView& t, const uint8_t* k
     tl.sync();  // the next op on this warp reads these writes
 }
 
-// The ops of the component led by op j, gathered by lane 0 from the lists of
-// j's free slot F and of every free slot the flow from F reaches (the flow
+// The ops of the component led by op j, gathered by one thread from the lists
+// of j's free slot F and of every free slot the flow from F reaches (the flow
 // pass's walk again: nothing in the component has run), their registrations
-// and list words set idle on the way; then sorted into index order by the
-// warp.  Returns their count, or 0 when there are more than DX_GATHER (their
-// ops then go to pend[1] for the component path).
-template <int T = 32>
-__device__ __noinline__ uint32_t dx_gather(const TableView& t, uint32_t j, uint32_t n0, const OpScratch& sc,
-                                           Ctl* ctl, uint32_t* s_ops, const Tile<T>& tl) {
+// and list words set idle on the way.  Returns their count; a count above
+// DX_GATHER: they are in pend[1], for the component path.
+__device__ __noinline__ uint32_t dx_gather_list(const TableView& t, uint32_t j, uint32_t n0, const OpScratch& sc,
+                                                Ctl* ctl, uint32_t* s_ops) {
     uint32_t g = 0;
-    if (tl.lane == 0) {
-        const uint64_t mask = t.mask;
-        uint64_t F = sc.op_slot[j];
-        uint64_t a = F, budget = mask;
-        uint64_t flow = 0;
-        for (;;) {
-            const uint32_t c = t.seg_cnt[F] & DX_CNT;
-            uint32_t x = t.seg_min[F];
-            if (c) {
-                t.seg_min[F] = IDLE;
-                t.seg_cnt[F] = 0;
-            }
-            for (uint32_t q = 0; q < c && x != IDLE; q++) {
-                if (x >= n0) {
-                    atomicOr(&ctl->err, ERR_SCRATCH);
-                    break;
-                }
-                const uint32_t nx = sc.op_word[x];
-                sc.op_word[x] = IDLE;
-                if (g == (uint32_t)DX_GATHER) {  // too many for this warp: all of them to the component path
-                    const uint32_t at = atomicAdd(&ctl->npend[1], (uint32_t)DX_GATHER);
-                    for (int i = 0; i < DX_GATHER; i++) sc.pend[1][at + i] = s_ops[i];
-                }
-                if (g < (uint32_t)DX_GATHER) s_ops[g] = x;
-                else sc.pend[1][atomicAdd(&ctl->npend[1], 1u)] = x;
-                ++g;
-                x = nx;
-            }
-            flow = flow + c - 1;
-            if (flow == 0) break;
-            const uint64_t at = dx_next_free(t, a + 1, budget);
-            if (at == NONE64) break;  // the flow pass found no wrap: not reached
-            a = at;
-            F = at & mask;
+    const uint64_t mask = t.mask;
+    uint64_t F = sc.op_slot[j];
+    uint64_t a = F, budget = mask;
+    uint64_t flow = 0;
+    for (;;) {
+        const uint32_t c = t.seg_cnt[F] & DX_CNT;
+        uint32_t x = t.seg_min[F];
+        if (c) {
+            t.seg_min[F] = IDLE;
+            t.seg_cnt[F] = 0;
         }
+        for (uint32_t q = 0; q < c && x != IDLE; q++) {
+            if (x >= n0) {
+                atomicOr(&ctl->err, ERR_SCRATCH);
+                break;
+            }
+            const uint32_t nx = sc.op_word[x];
+            sc.op_word[x] = IDLE;
+            if (g == (uint32_t)DX_GATHER) {  // too many for a warp: all of them to the component path
+                const uint32_t at = atomicAdd(&ctl->npend[1], (uint32_t)DX_GATHER);
+                for (int i = 0; i < DX_GATHER; i++) sc.pend[1][at + i] = s_ops[i];
+            }
+            if (g < (uint32_t)DX_GATHER) s_ops[g] = x;
+            else sc.pend[1][atomicAdd(&ctl->npend[1], 1u)] = x;
+            ++g;
+            x = nx;
+        }
+        flow = flow + c - 1;
+        if (flow == 0) break;
+        const uint64_t at = dx_next_free(t, a + 1, budget);
+        if (at == NONE64) break;  // the flow pass found no wrap: not reached
+        a = at;
+        F = at & mask;
     }
-    g = tl.shfl(g, 0);
-    tl.sync();
-    if (g > (uint32_t)DX_GATHER) return 0;
-    // index order: each lane ranks DX_GATHER / T entries
+    return g;
+}
+
+// The g <= DX_GATHER ops s_ops[0..g) into index order: each lane of the tile
+// ranks DX_GATHER / T of them.
+template <int T>
+__device__ __forceinline__ void dx_sort(uint32_t* s_ops, uint32_t g, const Tile<T>& tl) {
     constexpr int PER = DX_GATHER / T;
     const uint32_t lane = tl.lane;
     uint32_t v[PER], r[PER];
@@ -2526,6 +2899,19 @@ __device__ __noinline__ uint32_t dx_gather(const TableView& t, uint32_t j, uint3
     for (int u = 0; u < PER; u++)
         if (lane + T * u < g) s_ops[r[u]] = v[u];
     tl.sync();
+}
+
+// Both for the component led by op j, by a tile.  Returns the count, or 0 when
+// there are more than DX_GATHER.
+template <int T = 32>
+__device__ __forceinline__ uint32_t dx_gather(const TableView& t, uint32_t j, uint32_t n0, const OpScratch& sc,
+                                              Ctl* ctl, uint32_t* s_ops, const Tile<T>& tl) {
+    uint32_t g = 0;
+    if (tl.lane == 0) g = dx_gather_list(t, j, n0, sc, ctl, s_ops);
+    g = tl.shfl(g, 0);
+    tl.sync();
+    if (g > (uint32_t)DX_GATHER) return 0;
+    dx_sort<T>(s_ops, g, tl);
     return g;
 }
 
@@ -2624,6 +3010,296 @@ __device__ __noinline__ uint32_t dx_gather_q(const TableView& t, uint32_t j, uin
     return g;
 }
 
+// A component on a table without tombstones, all its ops at once.  Its ops
+// have keys that are not stored, so what they do to the slots from the lowest
+// home to the last free slot they fill has the closed form that fm_merge.cu
+// gives for a whole call: c(s) ops are carried across slot s, the group of
+// home h moves right by c(h) and turns once per op carried across it, and a
+// free slot takes the lowest index of the ops carried to it.  With at most 64
+// ops in index order the carried ones are a 64-bit mask: the lowest bit is
+// the one a free slot takes, and an op's rank among them is a bit count.
+// Metadata is read once and each record that moves is read and written once,
+// instead of one walk and one set of moves per op after the other.  A call of
+// 100K account pairs at load 0.8 lists about 10K components and 4K long
+// walks.
+constexpr uint32_t CF_SLOTS = 512;  // slots of a component run this way
+constexpr uint32_t CF_TAKE = 4;     // entries a warp takes at a time
+struct CfSmem {
+    uint32_t flags[CF_SLOTS];
+    uint16_t c[CF_SLOTS];    // ops that start at a slot (0/1), then c, then the destinations in order
+    uint16_t src[CF_SLOTS];  // what a slot holds afterwards: another slot, CF_OP | op, CF_STAYS
+    uint32_t val[DX_GATHER];  // the op giving each op's value
+    uint16_t home[DX_GATHER];
+    uint8_t rank[DX_GATHER];
+};
+constexpr uint32_t CF_OP = 0x8000u, CF_STAYS = 0xFFFFu;
+
+// Where entry `pos` of a group of m stored entries at home h (in slots of the
+// component) ends up in it; for op `mine` (>= 0) its own place.
+__device__ __forceinline__ uint32_t cf_turned(const CfSmem& s, unsigned long long alive, uint32_t h, uint32_t pos,
+                                              uint32_t m, uint32_t c, int mine) {
+    uint32_t size = m, seen = 0;
+    bool in = mine < 0;
+    for (unsigned long long b = alive; b; b &= b - 1) {
+        const int i = __ffsll((long long)b) - 1;
+        if (s.home[i] != h) continue;
+        const uint32_t r = s.rank[i] - seen;
+        if (in && size && r) pos = (pos + size - r % size) % size;
+        seen = s.rank[i];
+        if (i == mine) {
+            in = true;
+            pos = size;
+        }
+        ++size;
+    }
+    const uint32_t r = c - seen;
+    return r ? (pos + size - r % size) % size : pos;
+}
+
+// The g ops s_ops[0..g) (index order) of the component whose first free slot
+// is F.  False, with nothing written, when it spans more than CF_SLOTS.
+// Warp-uniform call.
+template <int KB, int VB>
+__device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restrict__ keys,
+                                    const uint8_t* __restrict__ vals, const uint32_t* s_ops, uint32_t g, uint64_t F,
+                                    const OpScratch& sc, CfSmem& s, ExecAcc& acc) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t m32 = (uint32_t)t.mask;
+    if (t.mask < 4 * CF_SLOTS) return false;
+    // the ops' homes from CF_SLOTS before F on
+    const uint32_t org = (uint32_t)F - CF_SLOTS;
+    uint32_t op[2], q[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const uint32_t i = lane + 32 * u;
+        op[u] = i < g ? s_ops[i] : IDLE;
+        q[u] = i < g ? (sc.op_pt[(uint64_t)op[u] * PT_MAX] - org) & m32 : 0xFFFFu;
+    }
+    const uint32_t top = __reduce_max_sync(FULL, max(q[0] == 0xFFFFu ? 0u : q[0], q[1] == 0xFFFFu ? 0u : q[1]));
+    if (top >= 2 * CF_SLOTS) return false;
+    const uint32_t low = __reduce_min_sync(FULL, min(q[0], q[1]));
+    // positions from S on, S aligned to four slots; the first home is at `al`
+    const uint32_t al = (org + low) & 3u;
+    const uint32_t S = org + low - al;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if (lane + 32 * u >= g) continue;
+        q[u] = q[u] - low + al;
+        s.home[lane + 32 * u] = (uint16_t)q[u];
+        s.val[lane + 32 * u] = op[u];
+    }
+    __syncwarp();
+    // repeats of a key: the first op inserts it with the last one's value
+    unsigned long long alive = g == 64 ? ~0ull : (1ull << g) - 1ull;
+    for (uint32_t i = 0; i + 1 < g; i++) {
+        if (!(alive >> i & 1ull)) continue;
+        const uint32_t hi = s.home[i];
+        unsigned long long same = (unsigned long long)__ballot_sync(FULL, q[0] == hi && lane < g) |
+                                  (unsigned long long)__ballot_sync(FULL, q[1] == hi && lane + 32 < g) << 32;
+        same &= alive & ~((2ull << i) - 1ull);
+        if (!same) continue;
+        RegKey<KB> ki;
+        ki.load(keys + (uint64_t)s_ops[i] * KB, KB);
+        bool eq[2] = {false, false};
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (!(same >> (lane + 32 * u) & 1ull)) continue;
+            RegKey<KB> k;
+            k.load(keys + (uint64_t)op[u] * KB, KB);
+            eq[u] = k.same(ki);
+        }
+        const unsigned long long dup = (unsigned long long)__ballot_sync(FULL, eq[0]) |
+                                       (unsigned long long)__ballot_sync(FULL, eq[1]) << 32;
+        if (dup) {
+            if (lane == 0) s.val[i] = s_ops[63 - __clzll((long long)dup)];
+            alive &= ~dup;
+        }
+    }
+    const uint32_t n = (uint32_t)__popcll(alive);
+    // the metadata, up to the n-th free slot
+    uint32_t len = 0, frees = 0;
+    while (frees < n) {
+        if (len == CF_SLOTS) return false;
+        const uint4 f = *reinterpret_cast<const uint4*>(t.flags + ((S + len + 4 * lane) & m32));
+        *reinterpret_cast<uint4*>(s.flags + len + 4 * lane) = f;
+        uint32_t fb = ~((f.x & 1u) | (f.y & 1u) << 1 | (f.z & 1u) << 2 | (f.w & 1u) << 3) & 15u;
+        if (len == 0 && lane == 0) fb &= 15u << al;
+        frees += __reduce_add_sync(FULL, (uint32_t)__popc(fb));
+        reinterpret_cast<uint2*>(s.c + len)[lane] = make_uint2(0u, 0u);
+        reinterpret_cast<uint2*>(s.src + len)[lane] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        len += 128;
+    }
+    if (top - low + al >= len) return false;  // never expected: every op's free slot is one of the n
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        if (alive >> (lane + 32 * u) & 1ull) s.c[q[u]] = 1;
+    __syncwarp();
+    // c at every slot and each op's rank among the ops carried across its home
+    unsigned long long pool = 0;
+    uint32_t done = 0, end = 0;
+    for (uint32_t w = 0; end == 0 && w < len; w += 32) {
+        const uint32_t fm = __ballot_sync(FULL, (s.flags[w + lane] & 1u) == 0u && w + lane >= al);
+        const uint32_t dm = __ballot_sync(FULL, s.c[w + lane] != 0);
+        uint32_t left = FULL;
+        uint32_t cl = (uint32_t)__popcll(pool);
+        for (;;) {
+            const uint32_t ev = (dm | (pool ? fm : 0u)) & left;
+            if (!ev) break;
+            const uint32_t e = __ffs(ev) - 1;
+            left = e == 31 ? 0u : FULL << (e + 1);
+            if (dm >> e & 1u) {
+                const unsigned long long here =
+                    ((unsigned long long)__ballot_sync(FULL, q[0] == w + e && lane < g) |
+                     (unsigned long long)__ballot_sync(FULL, q[1] == w + e && lane + 32 < g) << 32) & alive;
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const uint32_t i = lane + 32 * u;
+                    if (here >> i & 1ull) s.rank[i] = (uint8_t)__popcll(pool & ((1ull << i) - 1ull));
+                }
+                pool |= here;
+                done += (uint32_t)__popcll(here);
+            }
+            if ((fm >> e & 1u) && pool) pool &= pool - 1;
+            if (lane > e) cl = (uint32_t)__popcll(pool);
+            if (!pool && done == n) {
+                end = w + e + 1;
+                break;
+            }
+        }
+        __syncwarp();
+        s.c[w + lane] = (uint16_t)cl;
+    }
+    __syncwarp();
+    if (end == 0) return false;  // never expected
+    // where every entry goes
+    for (uint32_t x = lane; x < end; x += 32) {
+        const uint32_t f = s.flags[x];
+        const uint32_t d = f >> 4;
+        if (!(f & 1u) || x < al + d) continue;  // free, or its home lies before every op's
+        const uint32_t h = x - d, c = s.c[h];
+        if (c == 0) continue;
+        uint32_t i = 0, m = 1;
+        while (i < d && s.flags[x - i - 1] == mk_flag(ST_OCC, d - i - 1)) ++i;
+        while (x + m < end && s.flags[x + m] == mk_flag(ST_OCC, d + m)) ++m;
+        const uint32_t dst = x - i + c + cf_turned(s, alive, h, i, i + m, c, -1);
+        if (dst != x) s.src[dst] = (uint16_t)x;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const uint32_t i = lane + 32 * u;
+        if (!(alive >> i & 1ull)) continue;
+        uint32_t p = 0, m = 0;
+        for (;; ++p) {  // up to the first slot that is free or of a higher home
+            const uint32_t f = s.flags[q[u] + p];
+            if (!(f & 1u) || (f >> 4) < p) break;
+            m += (f >> 4) == p ? 1u : 0u;
+        }
+        const uint32_t c = s.c[q[u]];
+        s.src[q[u] + p - m + c + cf_turned(s, alive, q[u], 0, m, c, (int)i)] = (uint16_t)(CF_OP | i);
+    }
+    __syncwarp();
+    // the destinations, highest first
+    uint32_t cnt = 0;
+    for (int w = (int)((end - 1) & ~31u); w >= 0; w -= 32) {
+        const uint32_t x = (uint32_t)w + 31u - lane;
+        const bool mv = x < end && s.src[x] != CF_STAYS;
+        const uint32_t mm = __ballot_sync(FULL, mv);
+        if (mv) s.c[cnt + __popc(mm & ((1u << lane) - 1u))] = (uint16_t)x;
+        cnt += __popc(mm);
+    }
+    __syncwarp();
+    constexpr uint32_t BM = 16;
+    uint32_t md = 0;
+    for (uint32_t b = 0; b < cnt; b += BM) {
+        const uint32_t nb = min(BM, cnt - b);
+        uint32_t ks, vs, dst, dep;
+        {
+            const uint32_t x = s.c[b + min(lane, nb - 1u)], from = s.src[x];
+            if (from & CF_OP) {
+                const uint32_t i = from & ~CF_OP;
+                ks = s_ops[i] | MOVE_NEW;
+                vs = s.val[i] | MOVE_NEW;
+                dep = x - s.home[i];
+            } else {
+                ks = vs = (S + from) & m32;
+                dep = x - (from - (s.flags[from] >> 4));
+            }
+            dst = (S + x) & m32;
+            md = max(md, dep);
+        }
+        warp_move<KB, VB, BM>(t, keys, vals, nb, ks, vs, dst);
+        if (lane < nb) t.flags[dst] = mk_flag(ST_OCC, dep);
+        __syncwarp();
+    }
+    if (lane == 0) acc.claimed += n;
+    acc.maxd = max(acc.maxd, md);
+    return true;
+}
+
+// The component pass: on a table without tombstones, the entries the exec
+// pass listed, a warp each (cf_run).  An entry that spans too many slots is
+// passed on: its ops to pend[0], offset and count to op_pt (Ctl::nbig of
+// them), for the warp pass.  Bound by the latency of each entry's chain of
+// dependent reads (its lists, metadata, records), so it takes the registers
+// that let four blocks stay on an SM (two in the warp pass).
+template <int KB, int VB>
+__global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t* __restrict__ keys,
+                                                     const uint8_t* __restrict__ vals, uint32_t n0_arg, OpScratch sc,
+                                                     Ctl* ctl) {
+    __shared__ CfSmem s_cf[RBLOCK / 32];
+    __shared__ uint32_t s_ops[RBLOCK / 32][CF_TAKE][DX_GATHER];
+    __shared__ uint32_t s_tmp[RBLOCK / 32];
+    dx_wait_prev();
+    dx_let_next();
+    const uint32_t n = *(volatile const uint32_t*)&ctl->nlong[0];
+    if (n == 0 || !dx_clean(t, ctl)) return;  // block-uniform
+    const uint32_t n0 = cmp_n0(n0_arg, ctl);
+    const Tile<32> tl;
+    const uint32_t wi = threadIdx.x >> 5;
+    ExecAcc a;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    // CF_TAKE entries at a time: a lane each gathers their lists, at the same
+    // time, then the warp runs them one after another
+    for (uint32_t i0 = warp; i0 < n; i0 += CF_TAKE * warps) {
+        const uint32_t i = i0 + tl.lane * warps;
+        uint32_t mine = 0, F32 = 0;
+        if (tl.lane < CF_TAKE && i < n) {
+            const uint32_t item = sc.long_list[i];
+            F32 = (uint32_t)sc.op_slot[item & ~DX_ROOT];
+            if (item & DX_ROOT) {
+                mine = dx_gather_list(t, item & ~DX_ROOT, n0, sc, ctl, s_ops[wi][tl.lane]);
+                if (mine > (uint32_t)DX_GATHER) mine = 0;
+            } else {
+                s_ops[wi][tl.lane][0] = item;
+                mine = 1;
+            }
+        }
+        tl.sync();
+        for (uint32_t q = 0; q < CF_TAKE; q++) {
+            const uint32_t g = tl.shfl(mine, q), F = tl.shfl(F32, q);
+            if (g == 0) continue;
+            uint32_t* ops = s_ops[wi][q];
+            if (g > 1) dx_sort<32>(ops, g, tl);
+            if (!cf_run<KB, VB>(t, keys, vals, ops, g, F, sc, s_cf[wi], a)) {
+                uint32_t at = 0;
+                if (tl.lane == 0) {
+                    at = atomicAdd(&ctl->big_ops, g);
+                    const uint32_t k = atomicAdd(&ctl->nbig, 1u);
+                    sc.op_pt[(uint64_t)k * PT_MAX + 1] = at;
+                    sc.op_pt[(uint64_t)k * PT_MAX + 2] = g;
+                }
+                at = tl.shfl(at, 0);
+                for (uint32_t x = tl.lane; x < g; x += 32) sc.pend[0][at + x] = ops[x];
+            }
+            tl.sync();
+        }
+    }
+    block_add_count(ctl, a.claimed, s_tmp);
+    publish_rare(ctl, a.maxd, a.tomb, a.limit);
+}
+
 // The warp pass: a tile of T lanes per entry of the list the exec pass built
 // (T: 32, 16 or 8, chosen per record shape and load by the autotuner; a
 // narrower tile reads fewer slots per round trip but runs more entries at
@@ -2637,24 +3313,30 @@ __global__ void __launch_bounds__(RBLOCK, FM_P4_MIN_BLOCKS) k_dx_warp(TableView 
     __shared__ uint32_t s_ops[NT][DX_GATHER];
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     dx_wait_prev();
-    const uint32_t n = *(volatile const uint32_t*)&ctl->nlong[0];
+    const bool fresh = dx_clean(t, ctl);  // then: the entries the component pass left
+    const uint32_t n = *(volatile const uint32_t*)(fresh ? &ctl->nbig : &ctl->nlong[0]);
     if (n == 0) return;  // block-uniform
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
+    uint32_t* next = fresh ? &ctl->big_next : &ctl->nlong[1];
     const Tile<T> tl;
     const uint32_t ti = threadIdx.x / T;
     ExecAcc a;
-    // entries taken a warp's worth at a time from a counter (Ctl::nlong[1],
-    // zero at the start of the call): long entries do not hold up a static
+    // entries taken a warp's worth at a time from a counter (zero at the start
+    // of the call): long entries do not hold up a static
     // share of the list; all tiles of a warp loop together
     constexpr uint32_t TPW = 32 / T;
     for (;;) {
         uint32_t i0 = 0;
-        if ((threadIdx.x & 31u) == 0) i0 = atomicAdd(&ctl->nlong[1], TPW);
+        if ((threadIdx.x & 31u) == 0) i0 = atomicAdd(next, TPW);
         i0 = __shfl_sync(0xFFFFFFFFu, i0, 0);
         if (i0 >= n) break;
         const uint32_t i = i0 + (threadIdx.x & 31u) / T;
         uint32_t g = 0;  // a lone op, or a component's ops in index order
-        if (i < n) {
+        if (i < n && fresh) {
+            const uint32_t at = sc.op_pt[(uint64_t)i * PT_MAX + 1];
+            g = min(sc.op_pt[(uint64_t)i * PT_MAX + 2], (uint32_t)DX_GATHER);
+            for (uint32_t q = tl.lane; q < g; q += T) s_ops[ti][q] = sc.pend[0][at + q];
+        } else if (i < n) {
             const uint32_t item = sc.long_list[i];
             if (item & DX_ROOT) {
                 g = dx_gather<T>(t, item & ~DX_ROOT, n0, sc, ctl, s_ops[ti], tl);
@@ -2875,9 +3557,11 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
         uint32_t item = 0;
         bool defer = false;
         DxPlan p;
+        uint32_t h32 = 0;
         if (j < n0) {
             const uint64_t F = o.sc.op_slot[j];
             const uint64_t h = o.sc.op_pt[(uint64_t)j * PT_MAX];
+            h32 = (uint32_t)h;
             RegKey<KB> key;
             key.load(o.keys + (uint64_t)j * KB, KB);
             if (F != NONE64) {
@@ -2890,7 +3574,7 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
                     o.sc.op_word[j] = IDLE;
                 } else if (w == 1u) {
                     p.kind = -1;
-                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, false, sm.exec);
+                    if (lanes_ok) p = dx_plan<KB>(t, key, h, F, w0, sm.exec);
                     if (p.kind < 0) defer = true, item = j;
                     t.seg_min[F] = IDLE;
                     t.seg_cnt[F] = 0;
@@ -2902,7 +3586,7 @@ __device__ __noinline__ void q_iexec(const QOp& o, uint32_t c, uint32_t per, QSm
         }
         append(o.sc.long_list, &o.ctl->nlong[0], item, defer);
         __syncwarp();
-        dx_moves<KB, VB>(t, o.keys, o.vals, j, p, sm.exec, a);
+        dx_moves<KB, VB>(t, o.keys, o.vals, j, h32, p, sm.exec, a);
     }
     block_add_count(o.ctl, a.claimed, sm.tmp);
     publish_rare(o.ctl, a.maxd, a.tomb, a.limit);
@@ -3494,7 +4178,7 @@ constexpr Shape sh_of() {
 
 template <int KB, int VB>
 void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, cudaStream_t s) {
+                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, bool clean, cudaStream_t s) {
     if constexpr (KB == 0 || VB == 0) {
         return;
     } else {
@@ -3512,18 +4196,27 @@ void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, 
         }
         {
             KtScope kt(KC_INS_EXEC, s);
-            const unsigned ge = grid_for(nmax, 2);  // the resident blocks at most (two per SM)
-            launch_dependent(k_dx_exec<KB, VB>, ge, DX_THREADS, s, pdl, t, keys, vals, n0, sc, ctl);
+            const unsigned ge = grid_for(nmax, DX_BLOCKS);  // the resident blocks at most
+            const uint64_t warps = (uint64_t)num_sms() * FM_DC_BLOCKS * (DC_THREADS / 32);  // resident
+            const uint32_t opw = nmax <= warps * 4 ? 4 : (nmax <= warps * 8 ? 8 : (nmax <= warps * 16 ? 16 : 32));
+            const uint64_t per_block = (uint64_t)opw * (DC_THREADS / 32);
+            const unsigned gx = (unsigned)std::min<uint64_t>((nmax + per_block - 1) / per_block, (uint64_t)num_sms() * 64);
+            launch_dependent(k_dx_exec_clean<KB, VB>, gx,
+                             DC_THREADS, s, pdl, t, keys, vals, n0, opw, sc, ctl);
+            if (!clean)
+                launch_dependent(k_dx_exec<KB, VB>, ge, DX_THREADS, s, pdl, t, keys, vals, n0, sc, ctl);
         }
         {
             KtScope kt(KC_INS_LONG, s);
+            launch_dependent(k_dx_cf<KB, VB>, grid_for((uint64_t)nmax * 32, 4), RBLOCK, s, pdl, t, keys, vals, n0, sc,
+                             ctl);
             const int tw = tuned_ins_cfg(sh_of<KB, VB>(), (double)load).tile;
             const unsigned gwt = grid_for((uint64_t)nmax * tw, FM_P4_MIN_BLOCKS);
             if (tw == 8) launch_dependent(k_dx_warp<KB, VB, 8>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
             else if (tw == 16) launch_dependent(k_dx_warp<KB, VB, 16>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
             else launch_dependent(k_dx_warp<KB, VB, 32>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
         }
-        count_launches(4);
+        count_launches(clean ? 5 : 6);
     }
 }
 
@@ -3549,9 +4242,9 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 }
 
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
+                              const OpScratch& sc, Ctl* ctl, double load, bool clean, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, clean, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     return cudaGetLastError();
@@ -3560,7 +4253,7 @@ cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys,
 cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
                                   uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, false, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     return cudaGetLastError();

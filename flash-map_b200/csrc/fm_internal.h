@@ -126,8 +126,10 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 // ran and every op is left to launch_ins_comp at round 0; otherwise
 // Ctl::npend[1] ops (components too large for a warp) are left in pend[1]
 // for launch_ins_comp at round 1.
+// `clean`: the host knows that the table holds no tombstones, and the passes
+// for other tables are not launched (else both, and the device tells).
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s);
+                              const OpScratch& sc, Ctl* ctl, double load, bool clean, cudaStream_t s);
 // The same passes with the op count read from Ctl::n0 (a grouped call after
 // its precheck; nmax bounds it and sizes the grids) and no host step after
 // them: a call that found no free slot lists every op in pend[1], so
