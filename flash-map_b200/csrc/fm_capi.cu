@@ -109,7 +109,12 @@ struct DeviceGuard {
 // a mutating call while the current one runs).  Splitting a mutating batch
 // into consecutive pieces keeps the sequential semantics.
 constexpr uint64_t HOST_GET_PIECE = 1ull << 19;  // queries per get piece
-constexpr uint64_t HOST_MUT_PIECE = 1ull << 16;  // ops per insert/remove piece
+// An insert or remove piece: enough bytes that the copy of a piece outlasts
+// its call's launches and readback (a piece of 2^16 u64 pairs is 1 MB, about
+// 0.1 ms of copy against 0.1 ms of launches), at least 2^16 ops.
+constexpr uint64_t HOST_MUT_PIECE = 1ull << 16;
+constexpr uint64_t HOST_MUT_BYTES = 4ull << 20;
+uint64_t host_mut_piece(uint64_t record) { return std::max(HOST_MUT_PIECE, HOST_MUT_BYTES / std::max<uint64_t>(record, 1)); }
 
 struct GetCtx {
     cudaStream_t s[2] = {nullptr, nullptr};
@@ -364,7 +369,18 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
     *err_bits = 0;
     const fm::Shape sh = t->shape_for({d_k, d_v});
     const bool merge = insert && merge_wanted(t, sh, t->len.load(), n < OP_CHUNK ? n : OP_CHUNK);
-    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK, merge);
+    if (merge && t->cap <= fm::MG_SMALL_SLOTS && n <= fm::MG_SMALL_SLOTS) {
+        cudaError_t e = fm::launch_ins_small(t->view(), sh, d_k, d_v, (uint32_t)n, t->d_ctl, t->h_ctl, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
+        if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "merge insert", e);
+        if (!t->h_ctl->serial[0]) {
+            *out_count = t->h_ctl->total_count();
+            t->last_rounds = 0;
+            return FM_OK;
+        }
+    }
+    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK, merge && t->cap > fm::MG_SMALL_SLOTS);
     if (rc) return rc;
     fm::TableView v = t->view();
     for (uint64_t base = 0; base < n; base += OP_CHUNK) {
@@ -402,7 +418,7 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             e = fm::launch_rem_summary(v, t->sc, t->d_ctl, s);
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "round setup", e);
         }
-        if (merge && t->sc.carry && merge_wanted(t, sh, t->len.load() + total, m)) {
+        if (merge && t->cap > fm::MG_SMALL_SLOTS && t->sc.carry && merge_wanted(t, sh, t->len.load() + total, m)) {
             e = fm::launch_ins_merge(v, sh, kk, vv, m, t->sc, t->d_ctl, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -752,7 +768,7 @@ int host_pieces(fm_table* t, bool insert, const void* keys, const void* values, 
                 bool* limit) {
     *out = 0;
     *limit = false;
-    const uint64_t piece = n < HOST_MUT_PIECE ? n : HOST_MUT_PIECE;
+    const uint64_t piece = std::min(n, host_mut_piece(t->ksz + (insert ? t->vsz : 0)));
     const size_t kb = (size_t)piece * t->ksz, vb = insert ? (size_t)piece * t->vsz : 0;
     const size_t off_v = (kb + 255) & ~(size_t)255;
     const size_t half = (off_v + vb + 256) & ~(size_t)255;

@@ -99,7 +99,7 @@ constexpr uint64_t MG_CHUNK = 1024;       // slots per block of the scan
 constexpr uint64_t MG_MOVE_CHUNK = 1024;  // slots per block of the moves
 constexpr uint64_t MG_SMALL_SLOTS = 4096; // tables up to this size: one block does everything
 constexpr uint64_t MG_MIN_SLOTS = 1024;
-constexpr uint64_t MG_MAX_OPS = 1ull << 30;
+constexpr uint64_t MG_MAX_OPS = (1ull << 30) - 1;
 inline uint64_t mg_bytes(uint64_t mask) { return (mask + 1) * 4 + (mask + 1) / MG_CHUNK * 12; }
 
 enum Shape { SHAPE_8_8 = 0, SHAPE_32_128, SHAPE_32_64, SHAPE_32_32, SHAPE_8_32, SHAPE_GENERIC };
@@ -143,6 +143,12 @@ cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* k
 // path; otherwise every op is done.
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                              const OpScratch& sc, Ctl* ctl, cudaStream_t s);
+// The same for tables of MG_MIN_SLOTS to MG_SMALL_SLOTS, in one launch that
+// needs no scratch and no control block reset, leaves seg_min and seg_cnt as
+// they are, and writes the fields that the host reads after a call to `host`
+// (pinned memory).
+cudaError_t launch_ins_small(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                             Ctl* ctl, Ctl* host, cudaStream_t s);
 // Runs every remaining round starting at r in one block if the pending count
 // is at most TAIL_MAX; otherwise returns without touching anything.  With
 // handoff, rounds that stop progressing are left pending for the host

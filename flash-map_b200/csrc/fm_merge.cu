@@ -35,8 +35,10 @@
 //   fn, carry, slots             c at every slot (a scan of the functions
 //                                c -> max(a, c + b), MG_CHUNK slots a block)
 //   rank     (a thread per op)   each new op's rank among the ops carried
-//                                across its home
-//   old, new                     where every entry goes: seg_min[dest] = source
+//                                across its home (homes of several new ops)
+//   new      (a thread per op)   where each new op goes:
+//   old      (a thread per slot) where the stored entries go:
+//                                seg_min[dest] = source
 //   move     (a block per chunk) the records, once each, right to left between
 //                                two slots with c = 0 (entries move only right)
 // A call that outgrows a bound here (a home with too many ops or entries, a
@@ -46,6 +48,7 @@
 //
 // Bound by memory: the table's metadata is read about four times and each
 // record that moves is read and written once.
+#include <atomic>
 #include <type_traits>
 
 #include "fm_rounds.cuh"
@@ -58,13 +61,17 @@ constexpr uint32_t MG_LIST = 32;      // ops of one home a thread puts in order
 constexpr uint32_t MG_GROUP = 64;     // stored entries of one home on either side of one of them
 constexpr uint32_t MG_WALK = 1u << 14;  // slots a rank's walk looks back over
 constexpr uint32_t MG_EMPTY = 0x80000000u, MG_FRESH = 0x40000000u, MG_COUNT = 0x3FFFFFFFu;  // carry words
-constexpr uint32_t MG_SRC_OP = 0x80000000u;  // seg_min[dest]: the source is a new op
+constexpr uint32_t MG_SRC_OP = 0x80000000u;  // seg_min[dest]: the source is a new op,
+constexpr uint32_t MG_SRC_VAL = 0x40000000u; //   with another op's value
+constexpr uint32_t MG_MANY = 0x80000000u;    // seg_cnt[home]: the list has more than one op
 constexpr uint64_t MG_UPDATE = 1ull << 63;   // op_slot: an update of that slot
 constexpr int MG_THREADS = 256;
 
 // Per new op (op_pt, four words): the op giving its value, its rank among the
 // ops carried across its home, the number of ops on its home's list (first
-// op of the list only), the next op of the list.
+// op of the list only), the next op of the list.  seg_cnt[home] heads a list
+// (op + 1), with MG_MANY where it has several ops: the passes over the slots
+// read the list only there.
 struct __align__(16) MgOp {
     uint32_t val, rank, count, next;
 };
@@ -74,14 +81,14 @@ __device__ __forceinline__ bool mg_left(const Ctl* ctl) { return *(volatile cons
 
 // The passes are written for a crew of `step` threads of which this is number
 // `me`: the grid, or the one block of k_mg_small.
-template <int KB>
+template <int KB, bool RO>
 __device__ __forceinline__ void mg_find(const TableView& t, const uint8_t* __restrict__ keys, uint32_t n0,
                                         const OpScratch& sc, uint32_t me, uint32_t step) {
     MgOp* ops = mg_ops(sc);
     for (uint32_t j = me; j < n0; j += step) {
         RegKey<KB> key;
         const uint64_t h = home_of<KB>(t, keys, j, key);
-        const uint64_t x = get_probe_key<KB, true>(t, key, h);
+        const uint64_t x = get_probe_key<KB, RO>(t, key, h);
         if (x != NONE64) {
             sc.op_slot[j] = x | MG_UPDATE;
             sc.op_flag[j] = 0;
@@ -91,6 +98,7 @@ __device__ __forceinline__ void mg_find(const TableView& t, const uint8_t* __res
             const uint32_t before = atomicExch(&t.seg_cnt[h], j + 1u);  // 0: an empty list
             ops[j].next = before ? before - 1u : IDLE;
             sc.op_flag[j] = before ? 0 : 1;  // the first op of a list puts it in order
+            if (before) atomicOr(&sc.pend[0][(before - 1u) >> 5], 1u << ((before - 1u) & 31u));  // it is not alone
         }
     }
 }
@@ -120,11 +128,11 @@ __device__ __forceinline__ uint32_t mg_resolve(const TableView& t, const uint8_t
                     t.seg_min[x] = IDLE;
                 }
             } else if (sc.op_flag[j]) {
-                const uint32_t head = t.seg_cnt[at] - 1u;
-                if (head == j) {  // alone
+                if (!(sc.pend[0][j >> 5] >> (j & 31u) & 1u)) {  // alone
                     ops[j] = MgOp{j, 0u, 1u, IDLE};
                     ++fresh;
                 } else {
+                    const uint32_t head = t.seg_cnt[at] - 1u;
                     uint32_t list[MG_LIST], val[MG_LIST];
                     uint32_t c = 0, x = head;
                     bool over = false;
@@ -164,7 +172,7 @@ __device__ __forceinline__ uint32_t mg_resolve(const TableView& t, const uint8_t
                         }
                         for (uint32_t q = 0; q < u; q++)
                             ops[list[q]] = MgOp{val[q], 0u, q == 0 ? u : 0u, q + 1 < u ? list[q + 1] : IDLE};
-                        t.seg_cnt[at] = list[0] + 1u;
+                        t.seg_cnt[at] = (list[0] + 1u) | (u > 1 ? MG_MANY : 0u);
                         fresh += u;
                     }
                 }
@@ -191,8 +199,10 @@ __device__ __forceinline__ MgFn slot_fn(MgFn f, int fresh, bool empty) {
 }
 
 __device__ __forceinline__ int fresh_of(const OpScratch& sc, uint32_t w) {
-    return w ? (int)mg_ops(sc)[w - 1u].count : 0;
+    return w & MG_MANY ? (int)mg_ops(sc)[(w & ~MG_MANY) - 1u].count : (w ? 1 : 0);
 }
+// The first op of a list.
+__device__ __forceinline__ uint32_t first_of(uint32_t w) { return (w & ~MG_MANY) - 1u; }  // none: IDLE
 
 __device__ __forceinline__ MgFn warp_scan_fn(MgFn f) {  // inclusive
     const uint32_t lane = threadIdx.x & 31u;
@@ -321,17 +331,24 @@ __device__ __forceinline__ uint32_t mg_rank(const TableView& t, const MgOp* ops,
     const uint64_t mask = t.mask;
     int sum = 0, best = 0;
     uint64_t p = h + mask + 1;  // slots [p, h) are in the sum, unwrapped
-    for (uint32_t step = 0; step < MG_WALK; step += 4) {
-        const uint64_t b = (p - 1) & ~3ull;  // the quad that ends at or behind p
-        const uint4 q = *reinterpret_cast<const uint4*>(carry + (b & mask));
-        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+    for (uint32_t step = 0; step < MG_WALK; step += 8) {
+        // the eight slots that end at or behind p, with the lists that start there
+        const uint64_t b = (p - 1) & ~7ull;
+        const uint4* cp = reinterpret_cast<const uint4*>(carry + (b & mask));
+        const uint4* lp = reinterpret_cast<const uint4*>(t.seg_cnt + (b & mask));
+        const uint4 c0 = cp[0], c1 = cp[1], l0 = lp[0], l1 = lp[1];
+        const uint32_t w8[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const uint32_t n8[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
-        for (int l = 3; l >= 0; l--) {
+        for (int l = 7; l >= 0; l--) {
             if (b + l >= p) continue;
-            const uint32_t w = w4[l];
+            const uint32_t w = w8[l];
             if (w & MG_EMPTY) --sum;
             if (w & MG_FRESH) {
-                for (uint32_t x = t.seg_cnt[(b + l) & mask] - 1u; x < a; x = ops[x].next) ++sum;  // IDLE ends it
+                uint32_t x = first_of(n8[l]);
+                if (!(n8[l] & MG_MANY)) sum += x < a ? 1 : 0;
+                else
+                    for (; x < a; x = ops[x].next) ++sum;  // IDLE ends it
             }
             best = max(best, sum);
             if ((w & MG_COUNT) == 0 || best == (int)ch) return (uint32_t)best;
@@ -342,13 +359,17 @@ __device__ __forceinline__ uint32_t mg_rank(const TableView& t, const MgOp* ops,
     return 0;
 }
 
+// An op that is the only one of its home's list.
+__device__ __forceinline__ bool mg_one(const MgOp& op) { return op.count == 1u && op.next == IDLE; }
+
+// The ranks of the ops that share a home with others of the call.
 __device__ __forceinline__ void mg_ranks(const TableView& t, uint32_t n0, const OpScratch& sc, Ctl* ctl,
                                          const uint32_t* carry, uint32_t me, uint32_t step) {
     MgOp* ops = mg_ops(sc);
     bool over = false;
     for (uint32_t j = me; j < n0; j += step) {
         const uint64_t h = sc.op_slot[j];
-        if (h > t.mask) continue;  // an update or a repeat
+        if (h > t.mask || mg_one(ops[j])) continue;  // an update, a repeat, or for mg_new
         const uint32_t c = carry[h] & MG_COUNT;
         if (c) ops[j].rank = mg_rank(t, ops, carry, j, h, c, over);
     }
@@ -380,6 +401,8 @@ __device__ __forceinline__ uint32_t turned(const MgOp* ops, uint32_t head, uint3
 __device__ __forceinline__ void mg_old(const TableView& t, const OpScratch& sc, Ctl* ctl,
                                        const uint32_t* carry, uint64_t x) {
     const uint64_t mask = t.mask;
+    // what is carried across its home is carried on over every slot up to it
+    if ((carry[x] & MG_COUNT) == 0) return;
     const uint32_t f = t.flags[x];
     if (st_of(f) != ST_OCC) return;
     const uint32_t d = (uint32_t)dist_of(f);
@@ -398,18 +421,31 @@ __device__ __forceinline__ void mg_old(const TableView& t, const OpScratch& sc, 
         return;
     }
     const uint32_t w = t.seg_cnt[h];
-    const uint32_t to = turned(mg_ops(sc), w ? w - 1u : IDLE, i, i + m, c, IDLE);
+    const uint32_t to = turned(mg_ops(sc), first_of(w), i, i + m, c, IDLE);
     const uint64_t dst = (x - i + c + to) & mask;
     if (dst != x) t.seg_min[dst] = (uint32_t)x;
 }
 
-// Where every new op goes.
-__device__ __forceinline__ void mg_new(const TableView& t, uint32_t n0, const OpScratch& sc,
+// Where every new op goes, and the rank of an op that is alone on its home's
+// list (which the entries stored there turn by; with none stored it does not
+// matter).
+__device__ __forceinline__ void mg_new(const TableView& t, uint32_t n0, const OpScratch& sc, Ctl* ctl,
                                        const uint32_t* carry, uint32_t me, uint32_t step) {
     const uint64_t mask = t.mask;
+    MgOp* ops = mg_ops(sc);
+    bool over = false;
     for (uint32_t j = me; j < n0; j += step) {
         const uint64_t h = sc.op_slot[j];
         if (h > mask) continue;  // an update or a repeat
+        const uint32_t cw = carry[h];
+        const uint32_t c = cw & MG_COUNT;
+        MgOp op = ops[j];
+        const uint32_t code = j | MG_SRC_OP | (op.val != j ? MG_SRC_VAL : 0u);
+        const bool one = mg_one(op);
+        if (one && c == 0 && (cw & MG_EMPTY)) {
+            t.seg_min[h] = code;
+            continue;
+        }
         // the slots of this home's entries: behind those of lower homes, which
         // fill [h, s)
         uint32_t p = 0, m = 0;
@@ -430,10 +466,19 @@ __device__ __forceinline__ void mg_new(const TableView& t, uint32_t n0, const Op
                 }
             }
         }
-        const uint32_t c = carry[h] & MG_COUNT;
-        const uint32_t to = turned(mg_ops(sc), t.seg_cnt[h] - 1u, 0, m, c, j);
-        t.seg_min[(h + p - m + c + to) & mask] = j | MG_SRC_OP;
+        uint32_t to = 0;
+        if (!one) {
+            to = turned(ops, first_of(t.seg_cnt[h]), 0, m, c, j);
+        } else if (m) {  // at the end of the m, then turned by those carried across after it
+            if (c) {
+                op.rank = mg_rank(t, ops, carry, j, h, c, over);
+                ops[j].rank = op.rank;
+            }
+            to = m - (c - op.rank) % (m + 1);
+        }
+        t.seg_min[(h + p - m + c + to) & mask] = code;
     }
+    if (over) ctl->serial[0] = 1u;
 }
 
 // The moves of the slots from the first one with c = 0 at or after lo to the
@@ -532,9 +577,10 @@ __device__ __forceinline__ void mg_move(const TableView& t, const uint8_t* __res
                     const uint32_t s = sm.src[b + g / NP], c = g % NP;
                     const uint8_t* from;
                     if (s & MG_SRC_OP) {
-                        const uint32_t j = s & ~MG_SRC_OP;
-                        from = c < (uint32_t)NK ? keys + (uint64_t)j * KB + c * CK
-                                                : vals + (uint64_t)ops[j].val * VB + (c - NK) * CK;
+                        const uint32_t j = s & ~(MG_SRC_OP | MG_SRC_VAL);
+                        from = c < (uint32_t)NK
+                                   ? keys + (uint64_t)j * KB + c * CK
+                                   : vals + (uint64_t)(s & MG_SRC_VAL ? ops[j].val : j) * VB + (c - NK) * CK;
                     } else {
                         from = c < (uint32_t)NK ? t.keys + (uint64_t)s * KB + c * CK
                                                 : t.vals + (uint64_t)s * VB + (c - NK) * CK;
@@ -544,7 +590,13 @@ __device__ __forceinline__ void mg_move(const TableView& t, const uint8_t* __res
                 if (threadIdx.x < nb) {
                     const uint32_t s = sm.src[b + threadIdx.x];
                     const uint64_t dst = sm.dst[b + threadIdx.x];
-                    const uint64_t home = (s & MG_SRC_OP) ? sc.op_slot[s & ~MG_SRC_OP] : s - dist_of(t.flags[s]);
+                    uint64_t home;
+                    if (s & MG_SRC_OP) {  // from the key, which the move reads anyway
+                        RegKey<KB> key;
+                        home = home_of<KB>(t, keys, s & ~(MG_SRC_OP | MG_SRC_VAL), key);
+                    } else {
+                        home = s - dist_of(t.flags[s]);
+                    }
                     const uint32_t d = (uint32_t)((dst - home) & mask);
                     flag = mk_flag(ST_OCC, d);
                     md = max(md, d);
@@ -571,7 +623,7 @@ __device__ __forceinline__ void mg_move(const TableView& t, const uint8_t* __res
 template <int KB>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_find(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
                                                         OpScratch sc) {
-    mg_find<KB>(t, keys, n0, sc, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    mg_find<KB, true>(t, keys, n0, sc, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 template <int KB, int VB>
@@ -599,7 +651,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_old(TableView t, OpScratch sc
 __global__ void __launch_bounds__(MG_THREADS) k_mg_new(TableView t, uint32_t n0, OpScratch sc, Ctl* ctl,
                                                        const uint32_t* carry) {
     if (mg_left(ctl)) return;
-    mg_new(t, n0, sc, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    mg_new(t, n0, sc, ctl, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 template <int KB, int VB>
@@ -612,55 +664,98 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_move(TableView t, const uint8
     mg_move<KB, VB, MG_THREADS>(t, keys, vals, sc, ctl, carry, lo, lo + MG_MOVE_CHUNK, sm);
 }
 
-// All the passes on one block, for tables of at most MG_SMALL_SLOTS: such a
-// call is bound by launches, and its data stays in one SM's reach.
+// All the passes on one block, for tables of at most MG_SMALL_SLOTS.  Such a
+// call is bound by launches and by the latency of each pass's few reads, so
+// one launch does it all, with the table's metadata and everything else the
+// passes share in shared memory (160 KB at 4096 slots): 1000 account pairs
+// into 4096 slots took 37 us on one block over global memory.  The caller's
+// pinned control block is written directly (what the host reads of it).
 constexpr int MG_SMALL_THREADS = 1024;
+struct MgSmall {
+    uint64_t op_slot[MG_SMALL_SLOTS];
+    MgOp ops[MG_SMALL_SLOTS];
+    uint32_t flags[MG_SMALL_SLOTS], seg_min[MG_SMALL_SLOTS], seg_cnt[MG_SMALL_SLOTS], carry[MG_SMALL_SLOTS];
+    uint32_t many[MG_SMALL_SLOTS / 32];
+    uint8_t op_flag[MG_SMALL_SLOTS];
+};
 template <int KB, int VB>
-__global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView t, const uint8_t* __restrict__ keys,
+__global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView tg, const uint8_t* __restrict__ keys,
                                                                const uint8_t* __restrict__ vals, uint32_t n0,
-                                                               OpScratch sc, Ctl* ctl) {
+                                                               Ctl* ctl, Ctl* host) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ MgMoveSmem<MG_SMALL_THREADS> sm;
     __shared__ MgFn s_w[32];
-    __shared__ uint32_t s_tmp[MG_SMALL_THREADS / 32];
-    const uint32_t me = threadIdx.x, step = MG_SMALL_THREADS;
-    uint32_t* carry = sc.carry;
-    mg_find<KB>(t, keys, n0, sc, me, step);
-    __syncthreads();
-    const uint32_t fresh = mg_resolve<KB, VB>(t, keys, vals, n0, sc, ctl, me, step);
-    block_add_count(ctl, fresh, s_tmp);
-    __syncthreads();
-    if (mg_left(ctl)) return;  // block-uniform: the barrier is between the writes and this
-    const bool mine = me * 4 <= t.mask;  // MG_SMALL_SLOTS: four slots a thread
-    MgQuad q;
-    q.f = MgFn{0, 0};
-    if (mine) q.load(t, sc, me * 4);
-    MgFn total;
-    const MgFn ex = block_scan_fn(q.f, s_w, total);
-    if (total.b >= 0) {  // no slot stays EMPTY
-        if (me == 0) ctl->serial[0] = 1u;
-        return;
+    __shared__ uint32_t s_n[MG_SMALL_THREADS / 32];
+    __shared__ uint32_t s_ctl[sizeof(Ctl) / 4];
+    MgSmall& m = *reinterpret_cast<MgSmall*>(s_dyn);
+    Ctl* sctl = reinterpret_cast<Ctl*>(s_ctl);
+    const uint32_t me = threadIdx.x, step = MG_SMALL_THREADS, lane = me & 31u;
+    const uint32_t cap = (uint32_t)tg.mask + 1u;
+    TableView t = tg;
+    t.flags = m.flags, t.seg_min = m.seg_min, t.seg_cnt = m.seg_cnt;
+    OpScratch sc{};
+    sc.op_slot = m.op_slot, sc.op_flag = m.op_flag, sc.op_pt = reinterpret_cast<uint32_t*>(m.ops), sc.pend[0] = m.many;
+    if (me < MG_SMALL_SLOTS / 32) m.many[me] = 0;
+    for (uint32_t x = me; x < cap / 4; x += step) {
+        reinterpret_cast<uint4*>(m.flags)[x] = reinterpret_cast<const uint4*>(tg.flags)[x];
+        reinterpret_cast<uint4*>(m.seg_min)[x] = make_uint4(IDLE, IDLE, IDLE, IDLE);
+        reinterpret_cast<uint4*>(m.seg_cnt)[x] = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (mine) q.store(carry, me * 4, max(ex.a, total.a + ex.b));
+    if (me == 0) sctl->serial[0] = 0, sctl->dmax = ctl->dmax;
     __syncthreads();
-    mg_ranks(t, n0, sc, ctl, carry, me, step);
+    mg_find<KB, false>(t, keys, n0, sc, me, step);
     __syncthreads();
-    for (uint64_t x = me; x <= t.mask; x += step) mg_old(t, sc, ctl, carry, x);
-    mg_new(t, n0, sc, carry, me, step);
+    uint32_t fresh = mg_resolve<KB, VB>(t, keys, vals, n0, sc, sctl, me, step);
+    fresh = __reduce_add_sync(0xFFFFFFFFu, fresh);
+    if (lane == 0) s_n[me >> 5] = fresh;
     __syncthreads();
-    if (mg_left(ctl)) return;
-    mg_move<KB, VB, MG_SMALL_THREADS>(t, keys, vals, sc, ctl, carry, 0, t.mask + 1, sm);
+    bool left = mg_left(sctl);  // block-uniform, as below: a barrier between the writes and this
+    if (!left) {
+        const bool mine = me * 4 < cap;  // four slots a thread
+        MgQuad q;
+        q.f = MgFn{0, 0};
+        if (mine) q.load(t, sc, me * 4);
+        MgFn total;
+        const MgFn ex = block_scan_fn(q.f, s_w, total);
+        left = total.b >= 0;  // no slot stays EMPTY
+        if (!left) {
+            if (mine) q.store(m.carry, me * 4, max(ex.a, total.a + ex.b));
+            __syncthreads();
+            mg_ranks(t, n0, sc, sctl, m.carry, me, step);
+            __syncthreads();
+            mg_new(t, n0, sc, sctl, m.carry, me, step);
+            __syncthreads();
+            for (uint64_t x = me; x < cap; x += step) mg_old(t, sc, sctl, m.carry, x);
+            __syncthreads();
+            left = mg_left(sctl);
+        }
+    }
+    if (!left) {
+        mg_move<KB, VB, MG_SMALL_THREADS>(t, keys, vals, sc, sctl, m.carry, 0, cap, sm);
+        __syncthreads();
+        for (uint32_t x = me; x < cap / 4; x += step)
+            reinterpret_cast<uint4*>(tg.flags)[x] = reinterpret_cast<const uint4*>(m.flags)[x];
+    }
+    if (me < 32) {
+        const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, s_n[lane]);
+        if (me == 0) {
+            if (!left) ctl->dmax = sctl->dmax;
+            host->serial[0] = left ? 1u : 0u;
+            host->err = 0;
+            host->rounds = 0;
+            host->count = left ? 0u : n;
+            host->tomb_claimed = ctl->tomb_claimed;
+            __threadfence_system();
+        }
+        host->count_part[lane][0] = 0;
+    }
 }
+static_assert(COUNT_PARTS == 32, "a lane per count part");
 
 template <int KB, int VB>
 void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, const OpScratch& sc,
                  Ctl* ctl, cudaStream_t s) {
     const uint64_t cap = t.mask + 1;
-    if (cap <= MG_SMALL_SLOTS) {
-        KtScope kt(KC_INS_EXEC, s);
-        k_mg_small<KB, VB><<<1, MG_SMALL_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl);
-        count_launches(1);
-        return;
-    }
     uint32_t* carry = sc.carry;
     uint32_t* cin = carry + cap;
     int2* fn = reinterpret_cast<int2*>(cin + cap / MG_CHUNK);
@@ -668,6 +763,7 @@ void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, u
     const unsigned gc = (unsigned)(cap / MG_CHUNK);
     {
         KtScope kt(KC_INS_FIND, s);
+        cudaMemsetAsync(sc.pend[0], 0, ((size_t)n0 + 31) / 32 * 4, s);
         k_mg_find<KB><<<g, MG_THREADS, 0, s>>>(t, keys, n0, sc);
         k_mg_resolve<KB, VB><<<g, MG_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl);
     }
@@ -680,8 +776,8 @@ void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, u
     }
     {
         KtScope kt(KC_INS_EXEC, s);
-        k_mg_old<<<(unsigned)((cap + MG_THREADS - 1) / MG_THREADS), MG_THREADS, 0, s>>>(t, sc, ctl, carry);
         k_mg_new<<<g, MG_THREADS, 0, s>>>(t, n0, sc, ctl, carry);
+        k_mg_old<<<(unsigned)((cap + MG_THREADS - 1) / MG_THREADS), MG_THREADS, 0, s>>>(t, sc, ctl, carry);
     }
     {
         KtScope kt(KC_INS_LONG, s);
@@ -690,7 +786,38 @@ void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, u
     count_launches(9);
 }
 
+template <int KB, int VB>
+cudaError_t small_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, Ctl* ctl, Ctl* host,
+                        cudaStream_t s) {
+    static std::atomic<uint64_t> ready{0};  // devices on which the shared memory size is set, a bit each
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (!(ready.load() >> (dev & 63) & 1u)) {
+        e = cudaFuncSetAttribute(k_mg_small<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MgSmall));
+        if (e != cudaSuccess) return e;
+        if (dev < 64) ready.fetch_or(1ull << dev);
+    }
+    KtScope kt(KC_INS_EXEC, s);
+    k_mg_small<KB, VB><<<1, MG_SMALL_THREADS, sizeof(MgSmall), s>>>(t, keys, vals, n0, ctl, host);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 }  // namespace
+
+cudaError_t launch_ins_small(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                             Ctl* ctl, Ctl* host, cudaStream_t s) {
+    if (t.mask + 1 < MG_MIN_SLOTS || t.mask + 1 > MG_SMALL_SLOTS || n0 > MG_SMALL_SLOTS) return cudaErrorInvalidValue;
+    switch (sh) {
+        case SHAPE_8_8: return small_shape<8, 8>(t, keys, vals, n0, ctl, host, s);
+        case SHAPE_32_128: return small_shape<32, 128>(t, keys, vals, n0, ctl, host, s);
+        case SHAPE_32_64: return small_shape<32, 64>(t, keys, vals, n0, ctl, host, s);
+        case SHAPE_32_32: return small_shape<32, 32>(t, keys, vals, n0, ctl, host, s);
+        case SHAPE_8_32: return small_shape<8, 32>(t, keys, vals, n0, ctl, host, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
 
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                              const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
