@@ -235,6 +235,7 @@ struct fm_table {
     OpScratch sc{};
     size_t sc_bytes = 0;
     uint8_t* sc_base = nullptr;
+    uint32_t* d_carry = nullptr;  // merging inserts' words (ensure_carry)
     uint8_t* d_in = nullptr;  // host-API staging for mutating calls (two pieces)
     size_t d_in_cap = 0;
     cudaStream_t copy_stream = nullptr;  // prefetch of the next piece
@@ -276,28 +277,28 @@ struct TimerScope {
     ~TimerScope() { tl_timer = prev; }
 };
 
-int ensure_scratch(fm_table* t, uint64_t n, bool merge = false) {
-    if (t->sc.cap_ops >= n && (!merge || t->sc.carry)) return FM_OK;
-    merge = merge || t->sc.carry;
-    n = std::max(n, t->sc.cap_ops);
+// The merging inserts' words of a table, allocated once: captured graphs hold
+// their address, so they do not move when the scratch grows.  Without room
+// for them the calls run without the merge.
+void ensure_carry(fm_table* t) {
+    if (!t->d_carry && cudaMalloc((void**)&t->d_carry, fm::mg_bytes(t->mask)) != cudaSuccess) {
+        t->d_carry = nullptr;
+        cudaGetLastError();
+    }
+    t->sc.carry = t->d_carry;
+}
+
+int ensure_scratch(fm_table* t, uint64_t n) {
+    if (t->sc.cap_ops >= n) return FM_OK;
     // pend[0], pend[1] (u32) | op_slot (u64) | op_word (u32) | op_flag (u8) | op_pt (PT_MAX u32) |
     // long_list (u32) per op, then the component buffer and the remove chunk summaries (per table)
     const uint64_t per_op = 4 + 4 + 8 + 4 + 1 + 4 * fm::PT_MAX + 4;
     const uint64_t want = n + n / 4 + 1024;
-    size_t bytes = (size_t)(want * per_op + 10 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
+    const size_t bytes = (size_t)(want * per_op + 9 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
     if (t->sc_base) cudaFree(t->sc_base);
     t->sc_base = nullptr;
     t->sc = OpScratch{};
-    cudaError_t e = cudaErrorMemoryAllocation;
-    if (!fault_at(FM_FAULT_ALLOC)) {
-        if (merge && (e = cudaMalloc((void**)&t->sc_base, bytes + fm::mg_bytes(t->mask))) == cudaSuccess) {
-            bytes += fm::mg_bytes(t->mask);
-        } else {  // no room for the merge's words: the call runs without them
-            if (merge) cudaGetLastError();
-            merge = false;
-            e = cudaMalloc((void**)&t->sc_base, bytes);
-        }
-    }
+    cudaError_t e = dev_alloc((void**)&t->sc_base, bytes);
     if (e != cudaSuccess) return cuda_fail(FM_ERR_GPU_ALLOC, "scratch allocation", e);
     uint8_t* p = t->sc_base;
     auto carve = [&](size_t b) {
@@ -314,7 +315,7 @@ int ensure_scratch(fm_table* t, uint64_t n, bool merge = false) {
     t->sc.long_list = (uint32_t*)carve(want * 4);
     t->sc.comp = carve(fm::cmp_bytes(t->mask));
     t->sc.rsum = (uint32_t*)carve(4 * fm::rsum_words(t->mask));
-    if (merge) t->sc.carry = (uint32_t*)carve(fm::mg_bytes(t->mask));
+    t->sc.carry = t->d_carry;
     t->sc.cap_ops = want;
     t->sc_bytes = bytes;
     // op_word doubles as the insert inflow bound: idle value 0xFFFFFFFF.
@@ -380,8 +381,9 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             return FM_OK;
         }
     }
-    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK, merge && t->cap > fm::MG_SMALL_SLOTS);
+    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK);
     if (rc) return rc;
+    if (merge && t->cap > fm::MG_SMALL_SLOTS) ensure_carry(t);
     fm::TableView v = t->view();
     for (uint64_t base = 0; base < n; base += OP_CHUNK) {
         const uint32_t m = (uint32_t)((n - base) < OP_CHUNK ? (n - base) : OP_CHUNK);
@@ -691,6 +693,7 @@ void fm_destroy(fm_table* t) {
     cudaFree(t->d_ctl);
     if (t->h_ctl) cudaFreeHost(t->h_ctl);
     if (t->sc_base) cudaFree(t->sc_base);
+    if (t->d_carry) cudaFree(t->d_carry);
     if (t->d_in) cudaFree(t->d_in);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
@@ -1355,6 +1358,7 @@ struct fm_batch {
         bool remove = false;    // external: a remove
         bool get = false;       // external: a lookup
         bool direct = false;    // external insert: the direct passes (else the component path)
+        bool merge = false;     // external insert: the merge before them (tables without tombstones)
         double load = 0.0;      // external: the load it can reach (tuned tile width)
         uint32_t op = 0;        // external: the op
         fm::Shape shape = fm::SHAPE_GENERIC;
@@ -1464,6 +1468,12 @@ int queue_fill(fm_batch* b) {
         if (!need[i]) continue;
         int rc = ensure_scratch(b->tables[i], need[i]);
         if (rc) return rc;
+        // (a table whose plan has a merge; its address does not change)
+        for (const auto& st : b->qsteps)
+            if (st.merge && b->table_of[st.op] == i) {
+                ensure_carry(b->tables[i]);
+                break;
+            }
     }
     auto* q = reinterpret_cast<fm::QOp*>(b->h_desc + b->q_ops_off);
     for (size_t i = 0; i < b->ops.size(); i++) {
@@ -1589,6 +1599,8 @@ int queue_enqueue(fm_batch* b, cudaStream_t s, bool adaptive) {
                 continue;
             }
             e = fm::launch_grp_ins(st.shape, dg + st.ext, 1, h.n, fm::GRP_BEGIN, 0, 0, s);
+            if (e == cudaSuccess && st.merge && h.sc.carry)
+                e = fm::launch_ins_merge_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, s);
             if (e == cudaSuccess && st.direct) {
                 e = fm::launch_ins_direct_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, st.load, s);
                 if (e == cudaSuccess)
@@ -1638,6 +1650,15 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
     const uint32_t nops = (uint32_t)b->ops.size();
     std::vector<double> est(b->tables.size());
     for (size_t i = 0; i < b->tables.size(); i++) est[i] = (double)b->tables[i]->len.load();
+    // tables that may hold tombstones at this point of the batch (as planned;
+    // the merge's kernels see for themselves when they run)
+    std::vector<char> tombs(b->tables.size());
+    for (size_t i = 0; i < b->tables.size(); i++) tombs[i] = b->tables[i]->tombs.load();
+    auto merges = [&](const fm_op& o, uint32_t ti) {
+        const fm_table* t = o.table;
+        return !tombs[ti] && t->cap >= fm::MG_MIN_SLOTS && t->mask < (uint64_t)fm::DIST_MASK && o.n <= fm::MG_MAX_OPS &&
+               o.n * FM_MERGE_RATIO >= t->cap;
+    };
     if (b->qlanes) {
         // every op a device-driven step: a table's inserts and removes on its
         // lane in queue order; a lookup after the table's last write, on the
@@ -1677,6 +1698,8 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
             st.remove = o.kind == FM_OP_REMOVE;
             if (o.kind == FM_OP_INSERT) est[ti] = std::min(est[ti] + (double)o.n, cap);
             st.direct = est[ti] < FM_DIRECT_LOAD * cap;
+            st.merge = o.kind == FM_OP_INSERT && st.direct && merges(o, ti);
+            if (o.kind == FM_OP_REMOVE) tombs[ti] = 1;
             st.load = est[ti] / cap;
             st.ext = (uint32_t)b->qext_ops.size();
             b->qext_ops.push_back(i);
@@ -1753,6 +1776,7 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
                 fm_batch::QStep st;
                 st.external = true;
                 st.direct = est[ti] < FM_DIRECT_LOAD * cap;
+                st.merge = st.direct && merges(o, ti);
                 st.load = est[ti] / cap;
                 st.op = i;
                 st.shape = o.table->shape;
@@ -1762,6 +1786,7 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
                 continue;
             }
         }
+        if (o.kind == FM_OP_REMOVE) tombs[ti] = 1;
         if ((o.kind == FM_OP_REMOVE && o.n >= FM_QUEUE_REM_OPS) || (o.kind == FM_OP_GET && o.n >= FM_QUEUE_GET_OPS)) {
             flush();
             fm_batch::QStep st;

@@ -143,6 +143,12 @@ cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* k
 // path; otherwise every op is done.
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                              const OpScratch& sc, Ctl* ctl, cudaStream_t s);
+// The same with the op count read from Ctl::n0 (nmax bounds it and sizes the
+// grids) and no host step after it, for a table whose history the device
+// knows: on return the call is done and Ctl::n0 is 0, or (tombstones, or the
+// merge left the call) nothing has moved and the passes that follow run it.
+cudaError_t launch_ins_merge_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
+                                 uint32_t nmax, const OpScratch& sc, Ctl* ctl, cudaStream_t s);
 // The same for tables of MG_MIN_SLOTS to MG_SMALL_SLOTS, in one launch that
 // needs no scratch and no control block reset, leaves seg_min and seg_cnt as
 // they are, and writes the fields that the host reads after a call to `host`

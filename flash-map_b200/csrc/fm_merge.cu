@@ -79,6 +79,15 @@ __device__ __forceinline__ MgOp* mg_ops(const OpScratch& sc) { return reinterpre
 
 __device__ __forceinline__ bool mg_left(const Ctl* ctl) { return *(volatile const uint32_t*)&ctl->serial[0] != 0; }
 
+// For the kernels of a call: left, not for this path (tombstones; a call whose
+// history the host does not know), or empty.
+__device__ __forceinline__ uint32_t mg_n0(uint32_t n0, const Ctl* ctl) {
+    return n0 != CMP_N0_CTL ? n0 : *(volatile const uint32_t*)&ctl->n0;
+}
+__device__ __forceinline__ bool mg_skip(uint32_t n0, const Ctl* ctl) {
+    return mg_left(ctl) || *(volatile const uint32_t*)&ctl->tomb_claimed != 0 || mg_n0(n0, ctl) == 0;
+}
+
 // The passes are written for a crew of `step` threads of which this is number
 // `me`: the grid, or the one block of k_mg_small.
 template <int KB, bool RO>
@@ -268,9 +277,10 @@ __device__ __forceinline__ MgFn block_scan_fn(MgFn f, MgFn* s_w, MgFn& total) {
 }
 
 // The function of every chunk: a block per chunk, four slots a thread.
-__global__ void __launch_bounds__(MG_THREADS) k_mg_fn(TableView t, OpScratch sc, const Ctl* ctl, int2* fn) {
+__global__ void __launch_bounds__(MG_THREADS) k_mg_fn(TableView t, uint32_t n0, OpScratch sc, const Ctl* ctl,
+                                                      int2* fn) {
     __shared__ MgFn s_w[32];
-    if (mg_left(ctl)) return;
+    if (mg_skip(n0, ctl)) return;
     MgQuad q;
     q.load(t, sc, (uint64_t)blockIdx.x * MG_CHUNK + threadIdx.x * 4);
     MgFn total;
@@ -280,10 +290,10 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_fn(TableView t, OpScratch sc,
 
 // c at the start of every chunk (one block; the table is a ring: with fewer
 // new records than EMPTY slots the ring's function has the fixed point a).
-__global__ void __launch_bounds__(1024) k_mg_carry(uint64_t mask, Ctl* ctl, const int2* __restrict__ fn,
+__global__ void __launch_bounds__(1024) k_mg_carry(uint64_t mask, uint32_t n0, Ctl* ctl, const int2* __restrict__ fn,
                                                    uint32_t* __restrict__ cin) {
     __shared__ MgFn s_w[32];
-    if (mg_left(ctl)) return;  // block-uniform
+    if (mg_skip(n0, ctl)) return;  // block-uniform
     const uint64_t nch = (mask + 1) / MG_CHUNK;
     const uint64_t per = (nch + blockDim.x - 1) / blockDim.x;
     const uint64_t b0 = threadIdx.x * per, b1 = min(nch, b0 + per);
@@ -307,11 +317,11 @@ __global__ void __launch_bounds__(1024) k_mg_carry(uint64_t mask, Ctl* ctl, cons
 
 // c at every slot (a block per chunk), with what a walk over the slots needs
 // beside it: carry[s] = c(s) | MG_EMPTY | MG_FRESH (new ops start at s).
-__global__ void __launch_bounds__(MG_THREADS) k_mg_slots(TableView t, OpScratch sc, const Ctl* ctl,
+__global__ void __launch_bounds__(MG_THREADS) k_mg_slots(TableView t, uint32_t n0, OpScratch sc, const Ctl* ctl,
                                                          const uint32_t* __restrict__ cin,
                                                          uint32_t* carry) {
     __shared__ MgFn s_w[32];
-    if (mg_left(ctl)) return;
+    if (mg_skip(n0, ctl)) return;
     const uint64_t s0 = (uint64_t)blockIdx.x * MG_CHUNK + threadIdx.x * 4;
     MgQuad q;
     q.load(t, sc, s0);
@@ -622,8 +632,9 @@ __device__ __forceinline__ void mg_move(const TableView& t, const uint8_t* __res
 
 template <int KB>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_find(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
-                                                        OpScratch sc) {
-    mg_find<KB, true>(t, keys, n0, sc, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+                                                        OpScratch sc, const Ctl* ctl) {
+    if (mg_skip(n0, ctl)) return;
+    mg_find<KB, true>(t, keys, mg_n0(n0, ctl), sc, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 template <int KB, int VB>
@@ -631,37 +642,58 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_resolve(TableView t, const ui
                                                            const uint8_t* __restrict__ vals, uint32_t n0,
                                                            OpScratch sc, Ctl* ctl) {
     __shared__ uint32_t s_tmp[MG_THREADS / 32];
-    const uint32_t fresh = mg_resolve<KB, VB>(t, keys, vals, n0, sc, ctl, blockIdx.x * blockDim.x + threadIdx.x,
-                                              gridDim.x * blockDim.x);
+    // (serial[0] is set in this kernel: not a reason to leave it)
+    if (*(volatile const uint32_t*)&ctl->tomb_claimed != 0) return;
+    const uint32_t fresh = mg_resolve<KB, VB>(t, keys, vals, mg_n0(n0, ctl), sc, ctl,
+                                              blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     block_add_count(ctl, fresh, s_tmp);
 }
 
 __global__ void __launch_bounds__(MG_THREADS) k_mg_rank(TableView t, uint32_t n0, OpScratch sc, Ctl* ctl,
                                                         const uint32_t* carry) {
-    if (mg_left(ctl)) return;
-    mg_ranks(t, n0, sc, ctl, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if (mg_skip(n0, ctl)) return;
+    mg_ranks(t, mg_n0(n0, ctl), sc, ctl, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-__global__ void __launch_bounds__(MG_THREADS) k_mg_old(TableView t, OpScratch sc, Ctl* ctl,
+__global__ void __launch_bounds__(MG_THREADS) k_mg_old(TableView t, uint32_t n0, OpScratch sc, Ctl* ctl,
                                                        const uint32_t* carry) {
-    if (mg_left(ctl)) return;
+    if (mg_skip(n0, ctl)) return;
     mg_old(t, sc, ctl, carry, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x);  // a thread per slot
 }
 
 __global__ void __launch_bounds__(MG_THREADS) k_mg_new(TableView t, uint32_t n0, OpScratch sc, Ctl* ctl,
                                                        const uint32_t* carry) {
-    if (mg_left(ctl)) return;
-    mg_new(t, n0, sc, ctl, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if (mg_skip(n0, ctl)) return;
+    mg_new(t, mg_n0(n0, ctl), sc, ctl, carry, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 template <int KB, int VB>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_move(TableView t, const uint8_t* __restrict__ keys,
-                                                        const uint8_t* __restrict__ vals, OpScratch sc, Ctl* ctl,
-                                                        const uint32_t* carry) {
+                                                        const uint8_t* __restrict__ vals, uint32_t n0, OpScratch sc,
+                                                        Ctl* ctl, const uint32_t* carry) {
     __shared__ MgMoveSmem<MG_THREADS> sm;
-    if (mg_left(ctl)) return;
+    if (mg_skip(n0, ctl)) return;
     const uint64_t lo = (uint64_t)blockIdx.x * MG_MOVE_CHUNK;
     mg_move<KB, VB, MG_THREADS>(t, keys, vals, sc, ctl, carry, lo, lo + MG_MOVE_CHUNK, sm);
+}
+
+// After the passes of a call that has no host step: a call that was left has
+// its slot words set idle (k_mg_undo), then its flags and count taken back,
+// and one that is done has no ops for the passes that follow (k_mg_done).
+__global__ void __launch_bounds__(MG_THREADS) k_mg_undo(TableView t, const Ctl* ctl) {
+    if (*(volatile const uint32_t*)&ctl->tomb_claimed != 0 || !mg_left(ctl)) return;
+    for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x <= t.mask; x += (uint64_t)gridDim.x * blockDim.x)
+        t.seg_min[x] = IDLE, t.seg_cnt[x] = 0u;
+}
+__global__ void __launch_bounds__(32) k_mg_done(Ctl* ctl) {
+    if (*(volatile const uint32_t*)&ctl->tomb_claimed != 0) return;
+    const bool left = mg_left(ctl);
+    __syncwarp();
+    if (left) ctl->count_part[threadIdx.x][0] = 0;
+    if (threadIdx.x == 0) {
+        if (left) ctl->serial[0] = 0;
+        else ctl->n0 = 0;
+    }
 }
 
 // All the passes on one block, for tables of at most MG_SMALL_SLOTS.  Such a
@@ -753,37 +785,42 @@ __global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView tg, con
 static_assert(COUNT_PARTS == 32, "a lane per count part");
 
 template <int KB, int VB>
-void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, const OpScratch& sc,
-                 Ctl* ctl, cudaStream_t s) {
+void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
+                 const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
     const uint64_t cap = t.mask + 1;
     uint32_t* carry = sc.carry;
-    uint32_t* cin = carry + cap;
-    int2* fn = reinterpret_cast<int2*>(cin + cap / MG_CHUNK);
-    const unsigned g = grid_for(n0, 8);
+    int2* fn = reinterpret_cast<int2*>(carry + cap);  // before cin: one chunk's word would put it off 8 bytes
+    uint32_t* cin = reinterpret_cast<uint32_t*>(fn + cap / MG_CHUNK);
+    const unsigned g = grid_for(nmax, 8);
     const unsigned gc = (unsigned)(cap / MG_CHUNK);
     {
         KtScope kt(KC_INS_FIND, s);
-        cudaMemsetAsync(sc.pend[0], 0, ((size_t)n0 + 31) / 32 * 4, s);
-        k_mg_find<KB><<<g, MG_THREADS, 0, s>>>(t, keys, n0, sc);
+        cudaMemsetAsync(sc.pend[0], 0, ((size_t)nmax + 31) / 32 * 4, s);
+        k_mg_find<KB><<<g, MG_THREADS, 0, s>>>(t, keys, n0, sc, ctl);
         k_mg_resolve<KB, VB><<<g, MG_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl);
     }
     {
         KtScope kt(KC_INS_WALK, s);
-        k_mg_fn<<<gc, MG_THREADS, 0, s>>>(t, sc, ctl, fn);
-        k_mg_carry<<<1, 1024, 0, s>>>(t.mask, ctl, fn, cin);
-        k_mg_slots<<<gc, MG_THREADS, 0, s>>>(t, sc, ctl, cin, carry);
+        k_mg_fn<<<gc, MG_THREADS, 0, s>>>(t, n0, sc, ctl, fn);
+        k_mg_carry<<<1, 1024, 0, s>>>(t.mask, n0, ctl, fn, cin);
+        k_mg_slots<<<gc, MG_THREADS, 0, s>>>(t, n0, sc, ctl, cin, carry);
         k_mg_rank<<<g, MG_THREADS, 0, s>>>(t, n0, sc, ctl, carry);
     }
     {
         KtScope kt(KC_INS_EXEC, s);
         k_mg_new<<<g, MG_THREADS, 0, s>>>(t, n0, sc, ctl, carry);
-        k_mg_old<<<(unsigned)((cap + MG_THREADS - 1) / MG_THREADS), MG_THREADS, 0, s>>>(t, sc, ctl, carry);
+        k_mg_old<<<(unsigned)((cap + MG_THREADS - 1) / MG_THREADS), MG_THREADS, 0, s>>>(t, n0, sc, ctl, carry);
     }
     {
         KtScope kt(KC_INS_LONG, s);
-        k_mg_move<KB, VB><<<(unsigned)(cap / MG_MOVE_CHUNK), MG_THREADS, 0, s>>>(t, keys, vals, sc, ctl, carry);
+        k_mg_move<KB, VB><<<(unsigned)(cap / MG_MOVE_CHUNK), MG_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl, carry);
     }
     count_launches(9);
+    if (n0 == CMP_N0_CTL) {
+        k_mg_undo<<<grid_for(cap, 4), MG_THREADS, 0, s>>>(t, ctl);
+        k_mg_done<<<1, 32, 0, s>>>(ctl);
+        count_launches(2);
+    }
 }
 
 template <int KB, int VB>
@@ -819,19 +856,31 @@ cudaError_t launch_ins_small(const TableView& t, Shape sh, const uint8_t* keys, 
     }
 }
 
-cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                             const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
-    if (!sc.carry || t.mask + 1 < MG_MIN_SLOTS || t.mask >= (uint64_t)DIST_MASK || n0 > MG_MAX_OPS)
+namespace {
+cudaError_t merge_any(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
+                      const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
+    if (!sc.carry || t.mask + 1 < MG_MIN_SLOTS || t.mask >= (uint64_t)DIST_MASK || nmax > MG_MAX_OPS)
         return cudaErrorInvalidValue;
     switch (sh) {
-        case SHAPE_8_8: merge_shape<8, 8>(t, keys, vals, n0, sc, ctl, s); break;
-        case SHAPE_32_128: merge_shape<32, 128>(t, keys, vals, n0, sc, ctl, s); break;
-        case SHAPE_32_64: merge_shape<32, 64>(t, keys, vals, n0, sc, ctl, s); break;
-        case SHAPE_32_32: merge_shape<32, 32>(t, keys, vals, n0, sc, ctl, s); break;
-        case SHAPE_8_32: merge_shape<8, 32>(t, keys, vals, n0, sc, ctl, s); break;
+        case SHAPE_8_8: merge_shape<8, 8>(t, keys, vals, n0, nmax, sc, ctl, s); break;
+        case SHAPE_32_128: merge_shape<32, 128>(t, keys, vals, n0, nmax, sc, ctl, s); break;
+        case SHAPE_32_64: merge_shape<32, 64>(t, keys, vals, n0, nmax, sc, ctl, s); break;
+        case SHAPE_32_32: merge_shape<32, 32>(t, keys, vals, n0, nmax, sc, ctl, s); break;
+        case SHAPE_8_32: merge_shape<8, 32>(t, keys, vals, n0, nmax, sc, ctl, s); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                             const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
+    return merge_any(t, sh, keys, vals, n0, n0, sc, ctl, s);
+}
+
+cudaError_t launch_ins_merge_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
+                                 uint32_t nmax, const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
+    return merge_any(t, sh, keys, vals, CMP_N0_CTL, nmax, sc, ctl, s);
 }
 
 }  // namespace fm
