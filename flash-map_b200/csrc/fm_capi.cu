@@ -236,6 +236,7 @@ struct fm_table {
     size_t sc_bytes = 0;
     uint8_t* sc_base = nullptr;
     uint32_t* d_carry = nullptr;  // merging inserts' words (ensure_carry)
+    bool ctl_reset = true;        // d_ctl's per-call fields are zero (under mu; batches clear it)
     uint8_t* d_in = nullptr;  // host-API staging for mutating calls (two pieces)
     size_t d_in_cap = 0;
     cudaStream_t copy_stream = nullptr;  // prefetch of the next piece
@@ -389,8 +390,14 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
         const uint32_t m = (uint32_t)((n - base) < OP_CHUNK ? (n - base) : OP_CHUNK);
         const uint8_t* kk = d_k + base * t->ksz;
         const uint8_t* vv = d_v ? d_v + base * t->vsz : nullptr;
-        cudaError_t e = cudaMemsetAsync(t->d_ctl, 0, fm::CTL_CALL_BYTES, s);
+        cudaError_t e = cudaSuccess;
+        if (!t->ctl_reset) e = cudaMemsetAsync(t->d_ctl, 0, fm::CTL_CALL_BYTES, s);
         if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "round setup", e);
+        t->ctl_reset = false;
+        // after a wait for a call whose last kernel wrote h_ctl (publish_call)
+        auto published = [&] {
+            t->ctl_reset = !fm::ctl_left(t->h_ctl->serial[0], t->h_ctl->npend[1], t->h_ctl->nbig, t->h_ctl->err);
+        };
         uint32_t r = 0;
         uint32_t left = m;
         if (!insert) {
@@ -402,12 +409,13 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // and their bounded passes: it has no EMPTY slot for a probe to end at)
             const bool any_order = !t->claimed.load() && t->mask < (uint64_t)fm::DIST_MASK &&
                                    t->len.load() - total < t->cap;
-            e = any_order ? fm::launch_rem_take(v, sh, kk, m, t->d_ctl, s)
+            e = any_order ? fm::launch_rem_take(v, sh, kk, m, t->d_ctl, t->h_ctl, s)
                           : fm::launch_rem_direct(v, sh, kk, m, t->sc, t->d_ctl, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess && !any_order) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "remove", e);
+            if (any_order) published();
             if (t->h_ctl->err & fm::ERR_SCRATCH) return fail(FM_ERR_KERNEL_LAUNCH, "stale segment registration");
             r = t->h_ctl->serial[0] ? 0u : 1u;
             left = t->h_ctl->serial[0] ? m : t->h_ctl->npend[1];
@@ -421,11 +429,11 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "round setup", e);
         }
         if (merge && t->cap > fm::MG_SMALL_SLOTS && t->sc.carry && merge_wanted(t, sh, t->len.load() + total, m)) {
-            e = fm::launch_ins_merge(v, sh, kk, vv, m, t->sc, t->d_ctl, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+            e = fm::launch_ins_merge(v, sh, kk, vv, m, t->sc, t->d_ctl, t->h_ctl, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "merge insert", e);
+            published();
             if (!t->h_ctl->serial[0]) {
                 total += t->h_ctl->total_count();
                 t->last_rounds = 0;
@@ -452,9 +460,19 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // no free slot for some op, components too large for a warp) runs
             // on the component path
             const bool clean = t->mask >= 7 && t->mask < (uint64_t)fm::DIST_MASK && !t->tombs.load();
-            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, clean, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, clean, t->h_ctl, s);
+            if (e == cudaSuccess && !clean)
+                e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e == cudaSuccess && clean) {
+                published();
+                if (t->h_ctl->nbig) {  // components of too many slots for the component pass
+                    e = fm::launch_ins_direct_warp(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, s);
+                    if (e == cudaSuccess)
+                        e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+                    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                }
+            }
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "insert", e);
             if (t->h_ctl->err & fm::ERR_SCRATCH) return fail(FM_ERR_KERNEL_LAUNCH, "stale segment registration");
@@ -546,6 +564,7 @@ int run_rounds(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t* d_v,
     if (rc) {
         std::string msg = tl_err;
         recover(t, s);
+        t->ctl_reset = false;
         tl_err = msg;
         return rc;
     }
@@ -2178,6 +2197,7 @@ int fm_batch_capture(fm_batch* b, void* stream) {
 // The batch's removes may leave tombstones and its inserts claim them (what a
 // run did is known on the device only).
 static void batch_note_history(fm_batch* b) {
+    for (fm_table* t : b->tables) t->ctl_reset = false;
     for (const fm_op& o : b->ops)
         if (o.kind == FM_OP_REMOVE) o.table->tombs = true;
     for (const fm_op& o : b->ops)

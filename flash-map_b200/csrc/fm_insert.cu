@@ -3024,7 +3024,7 @@ __device__ __noinline__ uint32_t dx_gather_q(const TableView& t, uint32_t j, uin
 // walks.
 constexpr uint32_t CF_SLOTS = 512;  // slots of a component run this way
 constexpr uint32_t CF_TAKE = 4;     // entries a warp takes at a time
-struct CfSmem {
+struct __align__(16) CfSmem {  // moved in 16- and 8-byte pieces
     uint32_t flags[CF_SLOTS];
     uint16_t c[CF_SLOTS];    // ops that start at a slot (0/1), then c, then the destinations in order
     uint16_t src[CF_SLOTS];  // what a slot holds afterwards: another slot, CF_OP | op, CF_STAYS
@@ -3247,14 +3247,17 @@ __device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restric
 template <int KB, int VB>
 __global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t* __restrict__ keys,
                                                      const uint8_t* __restrict__ vals, uint32_t n0_arg, OpScratch sc,
-                                                     Ctl* ctl) {
+                                                     Ctl* ctl, Ctl* host) {
     __shared__ CfSmem s_cf[RBLOCK / 32];
     __shared__ uint32_t s_ops[RBLOCK / 32][CF_TAKE][DX_GATHER];
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     dx_wait_prev();
     dx_let_next();
     const uint32_t n = *(volatile const uint32_t*)&ctl->nlong[0];
-    if (n == 0 || !dx_clean(t, ctl)) return;  // block-uniform
+    if (n == 0 || !dx_clean(t, ctl)) {  // block-uniform
+        publish_call(ctl, host);
+        return;
+    }
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
     const Tile<32> tl;
     const uint32_t wi = threadIdx.x >> 5;
@@ -3298,6 +3301,7 @@ __global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t*
     }
     block_add_count(ctl, a.claimed, s_tmp);
     publish_rare(ctl, a.maxd, a.tomb, a.limit);
+    publish_call(ctl, host);
 }
 
 // The warp pass: a tile of T lanes per entry of the list the exec pass built
@@ -4177,8 +4181,20 @@ constexpr Shape sh_of() {
 }
 
 template <int KB, int VB>
+void warp_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
+                const OpScratch& sc, Ctl* ctl, float load, bool pdl, cudaStream_t s) {
+    if constexpr (KB != 0 && VB != 0) {
+        const int tw = tuned_ins_cfg(sh_of<KB, VB>(), (double)load).tile;
+        const unsigned gwt = grid_for((uint64_t)nmax * tw, FM_P4_MIN_BLOCKS);
+        if (tw == 8) launch_dependent(k_dx_warp<KB, VB, 8>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
+        else if (tw == 16) launch_dependent(k_dx_warp<KB, VB, 16>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
+        else launch_dependent(k_dx_warp<KB, VB, 32>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
+    }
+}
+
+template <int KB, int VB>
 void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, bool clean, cudaStream_t s) {
+                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, bool clean, Ctl* host, cudaStream_t s) {
     if constexpr (KB == 0 || VB == 0) {
         return;
     } else {
@@ -4209,14 +4225,10 @@ void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, 
         {
             KtScope kt(KC_INS_LONG, s);
             launch_dependent(k_dx_cf<KB, VB>, grid_for((uint64_t)nmax * 32, 4), RBLOCK, s, pdl, t, keys, vals, n0, sc,
-                             ctl);
-            const int tw = tuned_ins_cfg(sh_of<KB, VB>(), (double)load).tile;
-            const unsigned gwt = grid_for((uint64_t)nmax * tw, FM_P4_MIN_BLOCKS);
-            if (tw == 8) launch_dependent(k_dx_warp<KB, VB, 8>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
-            else if (tw == 16) launch_dependent(k_dx_warp<KB, VB, 16>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
-            else launch_dependent(k_dx_warp<KB, VB, 32>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
+                             ctl, clean ? host : nullptr);
+            if (!clean) warp_shape<KB, VB>(t, keys, vals, n0, nmax, sc, ctl, load, pdl, s);
         }
-        count_launches(clean ? 5 : 6);
+        count_launches(clean ? 4 : 6);
     }
 }
 
@@ -4242,18 +4254,28 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 }
 
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, bool clean, cudaStream_t s) {
+                              const OpScratch& sc, Ctl* ctl, double load, bool clean, Ctl* host, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, clean, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, clean, host, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                                   const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
+    KtScope kt(KC_INS_LONG, s);
+#define FM_CALL(K, V) warp_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, false, s)
+    FM_SHAPE_SWITCH(sh, FM_CALL)
+#undef FM_CALL
+    count_launches(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
                                   uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, false, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, false, nullptr, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     return cudaGetLastError();

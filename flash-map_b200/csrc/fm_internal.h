@@ -34,7 +34,8 @@ struct Ctl {
     uint32_t big_next;       //   the next of them to take
     uint32_t big_ops;        //   op indices they hold (pend[1])
     uint32_t exec_next;      // direct insert exec pass: the next op a warp takes
-    uint32_t pad_[7];        // count_part on a 32-byte boundary
+    uint32_t done;           // blocks that have reached the end of the call's last kernel (publish_call)
+    uint32_t pad_[6];        // count_part on a 32-byte boundary
     unsigned long long count;  // new keys (insert) / removed keys (remove), single-block kernels
     unsigned long long count_part[COUNT_PARTS][4];  // the same from grid kernels, [i][0] used
     // Persistent table facts (survive across calls, reset by clear):
@@ -52,6 +53,12 @@ constexpr uint32_t TOMB_MADE = 2u;     // a remove ran (it may have left tombsto
 constexpr size_t CTL_CALL_BYTES = 96 + 32 * COUNT_PARTS;  // npend .. count_part
 static_assert(offsetof(Ctl, count_part) % 32 == 0, "count parts in their own sectors");
 static_assert(offsetof(Ctl, dmax) == CTL_CALL_BYTES, "Ctl layout");
+
+// Whether a call's direct kernels left something for others (Ctl::serial[0],
+// npend[1], nbig, err): then the control block keeps its per-call fields.
+__host__ __device__ inline bool ctl_left(uint32_t serial0, uint32_t npend1, uint32_t nbig, uint32_t err) {
+    return (serial0 | npend1 | nbig | err) != 0;
+}
 
 // Op status codes written by device code (the FM_* values of the C ABI).
 constexpr int STATUS_OK = 0;
@@ -127,9 +134,15 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 // Ctl::npend[1] ops (components too large for a warp) are left in pend[1]
 // for launch_ins_comp at round 1.
 // `clean`: the host knows that the table holds no tombstones, and the passes
-// for other tables are not launched (else both, and the device tells).
+// for other tables are not launched (else both, and the device tells); then
+// `host` (pinned) takes the control block at the call's end, which is left
+// reset unless ctl_left, and what the component pass left (nbig) is left to
+// launch_ins_direct_warp.
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, bool clean, cudaStream_t s);
+                              const OpScratch& sc, Ctl* ctl, double load, bool clean, Ctl* host, cudaStream_t s);
+// The warp pass alone, for what the component pass left (Ctl::nbig).
+cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
+                                   const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s);
 // The same passes with the op count read from Ctl::n0 (a grouped call after
 // its precheck; nmax bounds it and sizes the grids) and no host step after
 // them: a call that found no free slot lists every op in pend[1], so
@@ -142,7 +155,7 @@ cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* k
 // moved: seg_min and seg_cnt are to be set idle and the call run by another
 // path; otherwise every op is done.
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                             const OpScratch& sc, Ctl* ctl, cudaStream_t s);
+                             const OpScratch& sc, Ctl* ctl, Ctl* host, cudaStream_t s);
 // The same with the op count read from Ctl::n0 (nmax bounds it and sizes the
 // grids) and no host step after it, for a table whose history the device
 // knows: on return the call is done and Ctl::n0 is 0, or (tombstones, or the
@@ -182,7 +195,8 @@ cudaError_t launch_rem_direct(const TableView& t, Shape sh, const uint8_t* keys,
                               Ctl* ctl, cudaStream_t s);
 // A whole remove call of n0 ops on a table with Ctl::tomb_claimed 0 and fewer
 // than 2^28 slots: the ops commute, one kernel, nothing left over.
-cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, cudaStream_t s);
+cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, Ctl* host,
+                            cudaStream_t s);
 // The same with the op count read from Ctl::n0 (nmax bounds it and sizes the
 // grids) and no host step after it: a call that found no EMPTY slot lists
 // every op in pend[1], so the rounds from round 1 complete the call either way.

@@ -670,11 +670,13 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_new(TableView t, uint32_t n0,
 template <int KB, int VB>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_move(TableView t, const uint8_t* __restrict__ keys,
                                                         const uint8_t* __restrict__ vals, uint32_t n0, OpScratch sc,
-                                                        Ctl* ctl, const uint32_t* carry) {
+                                                        Ctl* ctl, Ctl* host, const uint32_t* carry) {
     __shared__ MgMoveSmem<MG_THREADS> sm;
-    if (mg_skip(n0, ctl)) return;
-    const uint64_t lo = (uint64_t)blockIdx.x * MG_MOVE_CHUNK;
-    mg_move<KB, VB, MG_THREADS>(t, keys, vals, sc, ctl, carry, lo, lo + MG_MOVE_CHUNK, sm);
+    if (!mg_skip(n0, ctl)) {  // block-uniform
+        const uint64_t lo = (uint64_t)blockIdx.x * MG_MOVE_CHUNK;
+        mg_move<KB, VB, MG_THREADS>(t, keys, vals, sc, ctl, carry, lo, lo + MG_MOVE_CHUNK, sm);
+    }
+    publish_call(ctl, host);
 }
 
 // After the passes of a call that has no host step: a call that was left has
@@ -718,7 +720,7 @@ __global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView tg, con
     __shared__ MgMoveSmem<MG_SMALL_THREADS> sm;
     __shared__ MgFn s_w[32];
     __shared__ uint32_t s_n[MG_SMALL_THREADS / 32];
-    __shared__ uint32_t s_ctl[sizeof(Ctl) / 4];
+    __shared__ __align__(16) uint32_t s_ctl[sizeof(Ctl) / 4];
     MgSmall& m = *reinterpret_cast<MgSmall*>(s_dyn);
     Ctl* sctl = reinterpret_cast<Ctl*>(s_ctl);
     const uint32_t me = threadIdx.x, step = MG_SMALL_THREADS, lane = me & 31u;
@@ -786,7 +788,7 @@ static_assert(COUNT_PARTS == 32, "a lane per count part");
 
 template <int KB, int VB>
 void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                 const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
+                 const OpScratch& sc, Ctl* ctl, Ctl* host, cudaStream_t s) {
     const uint64_t cap = t.mask + 1;
     uint32_t* carry = sc.carry;
     int2* fn = reinterpret_cast<int2*>(carry + cap);  // before cin: one chunk's word would put it off 8 bytes
@@ -813,7 +815,7 @@ void merge_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, u
     }
     {
         KtScope kt(KC_INS_LONG, s);
-        k_mg_move<KB, VB><<<(unsigned)(cap / MG_MOVE_CHUNK), MG_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl, carry);
+        k_mg_move<KB, VB><<<(unsigned)(cap / MG_MOVE_CHUNK), MG_THREADS, 0, s>>>(t, keys, vals, n0, sc, ctl, host, carry);
     }
     count_launches(9);
     if (n0 == CMP_N0_CTL) {
@@ -858,15 +860,15 @@ cudaError_t launch_ins_small(const TableView& t, Shape sh, const uint8_t* keys, 
 
 namespace {
 cudaError_t merge_any(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                      const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
+                      const OpScratch& sc, Ctl* ctl, Ctl* host, cudaStream_t s) {
     if (!sc.carry || t.mask + 1 < MG_MIN_SLOTS || t.mask >= (uint64_t)DIST_MASK || nmax > MG_MAX_OPS)
         return cudaErrorInvalidValue;
     switch (sh) {
-        case SHAPE_8_8: merge_shape<8, 8>(t, keys, vals, n0, nmax, sc, ctl, s); break;
-        case SHAPE_32_128: merge_shape<32, 128>(t, keys, vals, n0, nmax, sc, ctl, s); break;
-        case SHAPE_32_64: merge_shape<32, 64>(t, keys, vals, n0, nmax, sc, ctl, s); break;
-        case SHAPE_32_32: merge_shape<32, 32>(t, keys, vals, n0, nmax, sc, ctl, s); break;
-        case SHAPE_8_32: merge_shape<8, 32>(t, keys, vals, n0, nmax, sc, ctl, s); break;
+        case SHAPE_8_8: merge_shape<8, 8>(t, keys, vals, n0, nmax, sc, ctl, host, s); break;
+        case SHAPE_32_128: merge_shape<32, 128>(t, keys, vals, n0, nmax, sc, ctl, host, s); break;
+        case SHAPE_32_64: merge_shape<32, 64>(t, keys, vals, n0, nmax, sc, ctl, host, s); break;
+        case SHAPE_32_32: merge_shape<32, 32>(t, keys, vals, n0, nmax, sc, ctl, host, s); break;
+        case SHAPE_8_32: merge_shape<8, 32>(t, keys, vals, n0, nmax, sc, ctl, host, s); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -874,13 +876,13 @@ cudaError_t merge_any(const TableView& t, Shape sh, const uint8_t* keys, const u
 }  // namespace
 
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                             const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
-    return merge_any(t, sh, keys, vals, n0, n0, sc, ctl, s);
+                             const OpScratch& sc, Ctl* ctl, Ctl* host, cudaStream_t s) {
+    return merge_any(t, sh, keys, vals, n0, n0, sc, ctl, host, s);
 }
 
 cudaError_t launch_ins_merge_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
                                  uint32_t nmax, const OpScratch& sc, Ctl* ctl, cudaStream_t s) {
-    return merge_any(t, sh, keys, vals, CMP_N0_CTL, nmax, sc, ctl, s);
+    return merge_any(t, sh, keys, vals, CMP_N0_CTL, nmax, sc, ctl, nullptr, s);
 }
 
 }  // namespace fm

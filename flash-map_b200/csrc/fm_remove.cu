@@ -569,13 +569,14 @@ __device__ __forceinline__ uint32_t rx_take(const TableView& t, const uint8_t* k
 // op with every thread of the SM resident keeps the most of them in flight.
 template <int KB>
 __global__ void __launch_bounds__(RBLOCK, 8) k_rx_take(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
-                                                       Ctl* ctl) {
+                                                       Ctl* ctl, Ctl* host) {
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     note_remove(ctl);
     uint32_t removed = 0;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x)
         removed += rx_take<KB>(t, keys, j);
     block_add_count(ctl, removed, s_tmp);
+    publish_call(ctl, host);
 }
 
 template <int KB>
@@ -886,16 +887,17 @@ cudaError_t launch_rem_direct(const TableView& t, Shape sh, const uint8_t* keys,
     return cudaGetLastError();
 }
 
-cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, cudaStream_t s) {
+cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, Ctl* host,
+                            cudaStream_t s) {
     KtScope kt(KC_REM_EXEC, s);
     const unsigned g = grid_for(n0, 8);
     switch (sh) {
         case SHAPE_8_8:
-        case SHAPE_8_32: k_rx_take<8><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
+        case SHAPE_8_32: k_rx_take<8><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl, host); break;
         case SHAPE_32_128:
         case SHAPE_32_64:
-        case SHAPE_32_32: k_rx_take<32><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
-        default: k_rx_take<0><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl); break;
+        case SHAPE_32_32: k_rx_take<32><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl, host); break;
+        default: k_rx_take<0><<<g, RBLOCK, 0, s>>>(t, keys, n0, ctl, host); break;
     }
     count_launches(1);
     return cudaGetLastError();
