@@ -2472,6 +2472,10 @@ int fm_autotune(int device, const char* cache_path) {
                 fm_table* bk_t = nullptr;
                 if ((rc = fm_create(cap, sk.k, sk.v, FM_HASH_IDENTITY, device, &bk_t)) != FM_OK) break;
                 rc = fm_copy(bk_t, t, s);
+                // one key removed (the first query's): the pass serves tables that
+                // may hold tombstones
+                uint64_t gone = 0;
+                if (rc == FM_OK) rc = fm_bulk_remove_device(bk_t, dq, 1, &gone, s);
                 const int tiles[] = {8, 16, 32};
                 float best_i = 1e30f;
                 int best_t = 32;

@@ -140,8 +140,12 @@ __global__ void __launch_bounds__(BLOCK) k_count(const uint32_t* __restrict__ fl
     }
 }
 
+// Bound by the latency of a query's dependent random reads (metadata, key,
+// value), so every thread the SM can hold should be one: 32 registers, eight
+// blocks per SM (4M account lookups at load 0.8, 2^24 slots: 307 us with the
+// 36 registers the compiler would take and seven blocks, 293 us with 32).
 template <int KB, int VB>
-__global__ void __launch_bounds__(BLOCK) k_get_thread(TableView t, const uint8_t* __restrict__ qkeys, uint64_t n,
+__global__ void __launch_bounds__(BLOCK, 8) k_get_thread(TableView t, const uint8_t* __restrict__ qkeys, uint64_t n,
                                                       uint8_t* __restrict__ out_vals,
                                                       uint8_t* __restrict__ out_found) {
 #if FM_GET_WCOPY
