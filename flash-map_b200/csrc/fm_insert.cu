@@ -2181,21 +2181,24 @@ __global__ void __launch_bounds__(RBLOCK) k_cmp_clean(TableView t, OpScratch sc)
 //         its own ops, and marks every later F it reaches (DX_ABS in seg_cnt)
 //         as part of this component, until the carry is 0.
 //   exec  (a thread per op)  an op alone at an unmarked F runs at once: its
-//         walk [home, F] from the metadata, the possible updates compared,
-//         the records moved two per round trip; a walk too long for one
-//         thread, and the leader of an unmarked F with c >= 2, go to the warp
-//         pass's list; the other ops wait for their component.
+//         walk [home, F] is planned on the thread (from the metadata, or the
+//         find pass's bits on tables without tombstones), the records moved by
+//         the warp; a walk too long for that, and the leader of an unmarked F
+//         with c >= 2, go to the list of the passes below; the other ops wait
+//         for their component.
 //   cf    (a warp per list entry; tables without tombstones)  a component
 //         gathers its ops from the lists of its free slots (the flow walk
 //         again), sorts them by index and does what they do at once; a long
 //         lone op likewise.
 //   warp  (a warp per list entry; other tables, and what cf leaves)  a long
 //         lone op runs as a tile walk; a component's ops one after another.
+// On tables without tombstones the find pass also tells updates apart (the key
+// is stored: nothing moves) and the flow pass writes them.
 // Components touch disjoint slots, so all of this runs at once.  A call that
 // finds an op with no free slot or a flow round the whole table leaves every
 // op to the component path (Ctl::serial[0]); a component with more ops than a
 // warp gathers leaves its ops to it (pend[1], Ctl::npend[1]).  Every
-// registration and list word is idle again when the four kernels end.
+// registration and list word is idle again when the kernels end.
 constexpr uint32_t DX_ABS = 0x80000000u;   // seg_cnt: the free slot is in an earlier slot's component
 constexpr uint32_t DX_CNT = 0x7FFFFFFFu;
 constexpr uint32_t DX_ROOT = 0x80000000u;  // warp-pass list entry: a component's leader
@@ -3020,8 +3023,8 @@ __device__ __noinline__ uint32_t dx_gather_q(const TableView& t, uint32_t j, uin
 // the one a free slot takes, and an op's rank among them is a bit count.
 // Metadata is read once and each record that moves is read and written once,
 // instead of one walk and one set of moves per op after the other.  A call of
-// 100K account pairs at load 0.8 lists about 10K components and 4K long
-// walks.
+// 100K account pairs into 2^24 slots at load 0.8 has about 6K components and
+// 7K walks that do not fit the bits.
 constexpr uint32_t CF_SLOTS = 512;  // slots of a component run this way
 constexpr uint32_t CF_TAKE = 4;     // entries a warp takes at a time
 struct __align__(16) CfSmem {  // moved in 16- and 8-byte pieces
