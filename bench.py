@@ -324,7 +324,7 @@ REMOVE_KERNELS = ("k_rem_p1", "k_rem_p2", "k_rem_p3", "k_rem_tail", "rem_group")
 # the same load factor and call size (the traffic summary under
 # profiles/ gives the command and the per-kernel figures); traffic grows with
 # the ops processed.
-NCU_TRAFFIC_PER_OP = {"insert": 2446.0, "get": 334.7, "remove": 515.2}
+NCU_TRAFFIC_PER_OP = {"insert": 2196.0, "get": 345.0, "remove": 209.4}
 
 
 class DeviceRun:
@@ -907,7 +907,7 @@ def main():
         peak, kind = read_peak()
         line["roofline"] = roofline_for(
             kt, INSERT_KERNELS, main_w.pairs, bpo["insert"], peak, kind,
-            "bulk_insert kernel set (k_dx_find, k_dx_flow, k_dx_exec, k_dx_warp, every call of the step; the step's "
+            "bulk_insert kernel set (k_dx_find, k_dx_flow, k_dx_exec_clean, k_dx_cf, every call of the step; the step's "
             "largest device-time share)", NCU_TRAFFIC_PER_OP["insert"])
         line["roofline_get"] = roofline_for(
             kt, ("k_get",), main_w.gets, bpo["get"], peak, kind, get_kernel_label(),
