@@ -235,6 +235,7 @@ struct fm_table {
     OpScratch sc{};
     size_t sc_bytes = 0;
     uint8_t* sc_base = nullptr;
+    uint64_t sc_gen = 0;          // counts the scratch's moves (captured graphs hold its addresses)
     uint32_t* d_carry = nullptr;  // merging inserts' words (ensure_carry)
     bool ctl_reset = true;        // d_ctl's per-call fields are zero (under mu; batches clear it)
     uint8_t* d_in = nullptr;  // host-API staging for mutating calls (two pieces)
@@ -299,6 +300,7 @@ int ensure_scratch(fm_table* t, uint64_t n) {
     if (t->sc_base) cudaFree(t->sc_base);
     t->sc_base = nullptr;
     t->sc = OpScratch{};
+    t->sc_gen += 1;
     cudaError_t e = dev_alloc((void**)&t->sc_base, bytes);
     if (e != cudaSuccess) return cuda_fail(FM_ERR_GPU_ALLOC, "scratch allocation", e);
     uint8_t* p = t->sc_base;
@@ -1399,6 +1401,7 @@ struct fm_batch {
     fm::QProf* d_prof = nullptr;     // per-phase timing (fm_batch_profile), one per phase
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<uint64_t> gens;  // per table: fm_table::sc_gen at the capture
     unsigned long long launches_per_run = 0;
     cudaStream_t last_stream = nullptr;
     bool pending = false;
@@ -2170,19 +2173,22 @@ int fm_batch_create(const fm_op* ops, uint32_t nops, fm_batch** out) {
 
 uint32_t fm_batch_waves(const fm_batch* b) { return b ? b->waves : 0; }
 
-int fm_batch_capture(fm_batch* b, void* stream) {
-    if (!b) return fail(FM_ERR_INVALID_ARG, "batch is NULL");
-    if (b->pending) return fail(FM_ERR_INVALID_ARG, "batch still running: call fm_batch_wait first");
-    DeviceGuard dg(b->device);
-    cudaStream_t s = (cudaStream_t)stream;
-    int rc = b->qmode ? queue_fill(b) : batch_fill(b);  // allocations (scratch growth) happen here, outside the capture
-    if (rc) return rc;
+// The moves of the tables' scratch so far.
+static std::vector<uint64_t> scratch_gens(const fm_batch* b) {
+    std::vector<uint64_t> g;
+    for (const fm_table* t : b->tables) g.push_back(t->sc_gen);
+    return g;
+}
+
+// Records the submission of a batch whose descriptors are filled into its
+// graph, in place of an earlier one.
+static int capture_filled(fm_batch* b, cudaStream_t s) {
     if (b->exec) cudaGraphExecDestroy(b->exec), b->exec = nullptr;
     if (b->graph) cudaGraphDestroy(b->graph), b->graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "begin capture", e);
     const unsigned long long l0 = fm::launch_count();
-    rc = b->qmode ? queue_enqueue(b, s, false) : batch_enqueue(b, s, false);
+    int rc = b->qmode ? queue_enqueue(b, s, false) : batch_enqueue(b, s, false);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(s, &g);
     if (rc) {
@@ -2194,7 +2200,29 @@ int fm_batch_capture(fm_batch* b, void* stream) {
     b->graph = g;
     e = cudaGraphInstantiate(&b->exec, g, 0);
     if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "graph instantiate", e);
+    b->gens = scratch_gens(b);
     return FM_OK;
+}
+
+// The graph again after a table's scratch has moved (a larger call on it, or
+// another batch's): its kernels hold the scratch addresses of the capture.
+// On a stream of its own, as the run's may be the legacy default stream.
+static int recapture(fm_batch* b) {
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "batch recapture stream", e);
+    const int rc = capture_filled(b, s);
+    cudaStreamDestroy(s);
+    return rc;
+}
+
+int fm_batch_capture(fm_batch* b, void* stream) {
+    if (!b) return fail(FM_ERR_INVALID_ARG, "batch is NULL");
+    if (b->pending) return fail(FM_ERR_INVALID_ARG, "batch still running: call fm_batch_wait first");
+    DeviceGuard dg(b->device);
+    int rc = b->qmode ? queue_fill(b) : batch_fill(b);  // allocations (scratch growth) happen here, outside the capture
+    if (rc) return rc;
+    return capture_filled(b, (cudaStream_t)stream);
 }
 
 // The batch's removes may leave tombstones and its inserts claim them (what a
@@ -2218,6 +2246,7 @@ int fm_batch_run(fm_batch* b, void* stream) {
     int rc;
     if (b->exec) {
         rc = b->qmode ? queue_fill(b) : batch_fill(b);
+        if (!rc && b->gens != scratch_gens(b)) rc = recapture(b);
         if (rc) return rc;
         cudaError_t e = cudaGraphLaunch(b->exec, s);
         if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "graph launch", e);
