@@ -350,6 +350,16 @@ void recover(fm_table* t, cudaStream_t s) {
     cudaStreamSynchronize(s);
 }
 
+// The table's history as the device has it, after a readback: the host's copy
+// can be behind (a clear() or a copy that ran ahead of a batch still in
+// flight).  Whether the table may hold tombstones.
+bool note_history(fm_table* t) {
+    const uint32_t h = t->h_ctl->tomb_claimed;
+    if (h) t->tombs = true;
+    if (h & fm::TOMB_CLAIMED) t->claimed = true;
+    return h != 0;
+}
+
 // Whether an insert of n ops runs as a merge: a table without tombstones, and
 // a call large enough beside the table that passes over all its slots cost
 // less than per-op work, and a load below FM_DIRECT_LOAD after it (beyond,
@@ -386,6 +396,7 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             t->last_rounds = 0;
             return FM_OK;
         }
+        note_history(t);
     }
     int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK);
     if (rc) return rc;
@@ -420,7 +431,7 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && fault_at(FM_FAULT_ROUND)) e = cudaErrorLaunchFailure;
             if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "remove", e);
-            if (any_order) published();
+            if (any_order) published();  // (serial[0]: a tombstone was claimed after all, nothing removed)
             if (t->h_ctl->err & fm::ERR_SCRATCH) return fail(FM_ERR_KERNEL_LAUNCH, "stale segment registration");
             r = t->h_ctl->serial[0] ? 0u : 1u;
             left = t->h_ctl->serial[0] ? m : t->h_ctl->npend[1];
@@ -444,6 +455,7 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
                 t->last_rounds = 0;
                 continue;
             }
+            note_history(t);
             // left undone before any record moved: the paths below run the call
             e = cudaMemsetAsync(t->d_seg_min, 0xFF, t->cap * 4, s);
             if (e == cudaSuccess) e = cudaMemsetAsync(t->d_seg_cnt, 0, t->cap * 4, s);
@@ -471,6 +483,7 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess && clean) {
                 published();
+                note_history(t);  // (tombstones after all: serial[0], the component path runs the call)
                 if (t->h_ctl->nbig) {  // components of too many slots for the component pass
                     e = fm::launch_ins_direct_warp(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, s);
                     if (e == cudaSuccess)

@@ -2655,17 +2655,21 @@ constexpr int DC_THREADS = 128;
 template <int KB, int VB>
 __global__ void __launch_bounds__(DC_THREADS, FM_DC_BLOCKS) k_dx_exec_clean(TableView t, const uint8_t* __restrict__ keys,
                                                                  const uint8_t* __restrict__ vals, uint32_t n0_arg,
-                                                                 uint32_t opw, OpScratch sc, Ctl* ctl) {
+                                                                 uint32_t opw, bool alone, OpScratch sc, Ctl* ctl) {
     constexpr uint32_t FULL = 0xFFFFFFFFu, OWN = 0x2000u;  // list: lane << 8 | bit, OWN: the op's own entry
     constexpr uint32_t BM = FM_DC_BATCH;
     __shared__ uint16_t s_list[DC_THREADS / 32][32 * (DX_LCH + 1) + 1];
     __shared__ uint32_t s_tmp[DC_THREADS / 32];
     dx_wait_prev();
     dx_let_next();
-    if (!dx_clean(t, ctl)) return;  // block-uniform
+    const bool clean = dx_clean(t, ctl);  // block-uniform
+    // alone: k_dx_exec is not launched beside it.  Tombstones that the host
+    // did not know of then send every op to the component path.
+    if (!clean && !alone) return;
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
     const bool to_pend = n0_arg == CMP_N0_CTL;  // as k_dx_exec
-    const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;
+    const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0 || !clean;
+    if (!clean && blockIdx.x == 0 && threadIdx.x == 0) ctl->serial[0] = 1u;
     const uint32_t lane = threadIdx.x & 31u, m32 = (uint32_t)t.mask;
     uint16_t* list = s_list[threadIdx.x >> 5];
     uint32_t claimed = 0, md = 0;
@@ -4221,7 +4225,7 @@ void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, 
             const uint64_t per_block = (uint64_t)opw * (DC_THREADS / 32);
             const unsigned gx = (unsigned)std::min<uint64_t>((nmax + per_block - 1) / per_block, (uint64_t)num_sms() * 64);
             launch_dependent(k_dx_exec_clean<KB, VB>, gx,
-                             DC_THREADS, s, pdl, t, keys, vals, n0, opw, sc, ctl);
+                             DC_THREADS, s, pdl, t, keys, vals, n0, opw, clean, sc, ctl);
             if (!clean)
                 launch_dependent(k_dx_exec<KB, VB>, ge, DX_THREADS, s, pdl, t, keys, vals, n0, sc, ctl);
         }

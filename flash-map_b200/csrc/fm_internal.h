@@ -134,8 +134,9 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 // Ctl::npend[1] ops (components too large for a warp) are left in pend[1]
 // for launch_ins_comp at round 1.
 // `clean`: the host knows that the table holds no tombstones, and the passes
-// for other tables are not launched (else both, and the device tells); then
-// `host` (pinned) takes the control block at the call's end, which is left
+// for other tables are not launched (else both, and the device tells; should
+// it hold some after all, serial[0] leaves every op as above); then `host`
+// (pinned) takes the control block at the call's end, which is left
 // reset unless ctl_left, and what the component pass left (nbig) is left to
 // launch_ins_direct_warp.
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
@@ -153,7 +154,8 @@ cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* k
 // (compile-time record shapes, MG_MIN_SLOTS to 2^28 slots, OpScratch::carry).
 // On return (stream-ordered) Ctl::serial[0] set means that no record has
 // moved: seg_min and seg_cnt are to be set idle and the call run by another
-// path; otherwise every op is done.
+// path; otherwise every op is done.  (A table that turns out to hold
+// tombstones is left too, and by launch_ins_small.)
 cudaError_t launch_ins_merge(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                              const OpScratch& sc, Ctl* ctl, Ctl* host, cudaStream_t s);
 // The same with the op count read from Ctl::n0 (nmax bounds it and sizes the
@@ -193,8 +195,10 @@ cudaError_t launch_ins_comp(const TableView& t, Shape sh, const uint8_t* keys, c
 // warp) are left in pend[1] for the rounds from round 1.
 cudaError_t launch_rem_direct(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, const OpScratch& sc,
                               Ctl* ctl, cudaStream_t s);
-// A whole remove call of n0 ops on a table with Ctl::tomb_claimed 0 and fewer
-// than 2^28 slots: the ops commute, one kernel, nothing left over.
+// A whole remove call of n0 ops on a table without TOMB_CLAIMED in
+// Ctl::tomb_claimed and of at most 2^27 slots: the ops commute, one kernel,
+// nothing left over.  Should the bit be set after all, serial[0] leaves every
+// op to the rounds from round 0.
 cudaError_t launch_rem_take(const TableView& t, Shape sh, const uint8_t* keys, uint32_t n0, Ctl* ctl, Ctl* host,
                             cudaStream_t s);
 // The same with the op count read from Ctl::n0 (nmax bounds it and sizes the

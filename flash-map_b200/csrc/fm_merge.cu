@@ -632,8 +632,12 @@ __device__ __forceinline__ void mg_move(const TableView& t, const uint8_t* __res
 
 template <int KB>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_find(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
-                                                        OpScratch sc, const Ctl* ctl) {
-    if (mg_skip(n0, ctl)) return;
+                                                        OpScratch sc, Ctl* ctl) {
+    if (mg_skip(n0, ctl)) {
+        // a call that the host sent here for a table with tombstones: left
+        if (n0 != CMP_N0_CTL && blockIdx.x == 0 && threadIdx.x == 0) ctl->serial[0] = 1u;
+        return;
+    }
     mg_find<KB, true>(t, keys, mg_n0(n0, ctl), sc, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -728,6 +732,11 @@ __global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView tg, con
     Ctl* sctl = reinterpret_cast<Ctl*>(s_ctl);
     const uint32_t me = threadIdx.x, step = MG_SMALL_THREADS, lane = me & 31u;
     const uint32_t cap = (uint32_t)tg.mask + 1u;
+    const uint32_t history = ctl->tomb_claimed;
+    if (history != 0) {  // block-uniform: a table with tombstones is not for this path
+        if (me == 0) host->serial[0] = 1u, host->err = 0, host->tomb_claimed = history;
+        return;
+    }
     TableView t = tg;
     t.flags = m.flags, t.seg_min = m.seg_min, t.seg_cnt = m.seg_cnt;
     OpScratch sc{};
@@ -781,7 +790,7 @@ __global__ void __launch_bounds__(MG_SMALL_THREADS) k_mg_small(TableView tg, con
             host->err = 0;
             host->rounds = 0;
             host->count = left ? 0u : n;
-            host->tomb_claimed = ctl->tomb_claimed;
+            host->tomb_claimed = history;
             __threadfence_system();
         }
         host->count_part[lane][0] = 0;

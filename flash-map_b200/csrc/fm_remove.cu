@@ -571,10 +571,15 @@ template <int KB>
 __global__ void __launch_bounds__(RBLOCK, 8) k_rx_take(TableView t, const uint8_t* __restrict__ keys, uint32_t n0,
                                                        Ctl* ctl, Ctl* host) {
     __shared__ uint32_t s_tmp[RBLOCK / 32];
-    note_remove(ctl);
     uint32_t removed = 0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x)
-        removed += rx_take<KB>(t, keys, j);
+    if (*(volatile const uint32_t*)&ctl->tomb_claimed & TOMB_CLAIMED) {  // block-uniform
+        // the host's copy of the history was behind: every op is left to the rounds
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->serial[0] = 1u;
+    } else {
+        note_remove(ctl);
+        for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n0; j += gridDim.x * blockDim.x)
+            removed += rx_take<KB>(t, keys, j);
+    }
     block_add_count(ctl, removed, s_tmp);
     publish_call(ctl, host);
 }
