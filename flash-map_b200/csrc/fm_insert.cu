@@ -2909,9 +2909,11 @@ __device__ __forceinline__ void dx_sort(uint32_t* s_ops, uint32_t g, const Tile<
 }
 
 // Both for the component led by op j, by a tile.  Returns the count, or 0 when
-// there are more than DX_GATHER.
+// there are more than DX_GATHER.  Out of line: in line it took registers from
+// the walks of the warp pass, whose loads then waited for one another (1000
+// account pairs into 2^23 slots at load 0.92: 261 against 375 us).
 template <int T = 32>
-__device__ __forceinline__ uint32_t dx_gather(const TableView& t, uint32_t j, uint32_t n0, const OpScratch& sc,
+__device__ __noinline__ uint32_t dx_gather(const TableView& t, uint32_t j, uint32_t n0, const OpScratch& sc,
                                               Ctl* ctl, uint32_t* s_ops, const Tile<T>& tl) {
     uint32_t g = 0;
     if (tl.lane == 0) g = dx_gather_list(t, j, n0, sc, ctl, s_ops);
