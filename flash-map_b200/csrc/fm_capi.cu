@@ -4,6 +4,7 @@
 // src/gpu.rs (bajpainaman/flash-map 0.5.0); see include/flashmap_b200.h.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -376,6 +377,29 @@ bool merge_wanted(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n) {
            (double)(len + n) < FM_DIRECT_LOAD * (double)t->cap;
 }
 
+// Whether a direct insert of n ops into a table without tombstones runs on
+// the passes for such tables.  They lose where the component pass leaves
+// entries of more than its 512 slots to the warp pass: that is a second wait,
+// and both passes for those entries.  A walk at load r is longer than x slots
+// with a probability of about exp(-x (1 - r)^2); with e = n exp(-450 (1 -
+// reach)^2) as the measure of it, these passes took, beside the general ones,
+// 0.87-0.93 of the time on average for e below 0.3 (one entry too long in an
+// eighth of the calls), 1.03 from 0.3 to 1, 1.2 from 3 to 100 (414 calls: u64,
+// 32/32 and account pairs, 2^13 to 2^23 slots, loads 0.80 to 0.94, 4 to 100,000
+// ops).  Account pairs into 2^20 slots: load 0.80, 1000 ops 79 against 120 us;
+// load 0.85, 256 ops 76 against 96, 10,000 ops 160 against 308; load 0.90, 256
+// ops 195 against 160, 10,000 ops 875 against 791.  The component pass needs
+// 1024 slots: of a smaller table it left every new key (64 to 256 slots: 62
+// against 36 us a call).
+#ifndef FM_CLEAN_WALK
+#define FM_CLEAN_WALK 450.0
+#endif
+bool clean_passes_pay(const fm_table* t, double reach, uint64_t n) {
+    const double gap = 1.0 - reach;
+    return t->cap >= fm::CLEAN_MIN_SLOTS && t->mask < (uint64_t)fm::DIST_MASK && gap > 0.0 &&
+           (double)n * std::exp(-FM_CLEAN_WALK * gap * gap) < 0.25;
+}
+
 // The round driver shared by insert and remove.  Each pass launches two
 // grid-wide rounds and the single-block tail back to back, then reads the
 // control block once: a zero pending count for the next round means done.
@@ -476,8 +500,9 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // index order per component; what the kernels leave (a table with
             // no free slot for some op, components too large for a warp) runs
             // on the component path
-            const bool clean = t->mask >= 7 && t->mask < (uint64_t)fm::DIST_MASK && !t->tombs.load();
-            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, clean, t->h_ctl, s);
+            const bool clean = !t->tombs.load() && clean_passes_pay(t, reach, m);
+            e = fm::launch_ins_direct(v, sh, kk, vv, m, t->sc, t->d_ctl, reach, clean ? fm::DX_ALONE : fm::DX_GENERAL,
+                                      t->h_ctl, s);
             if (e == cudaSuccess && !clean)
                 e = cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1396,6 +1421,7 @@ struct fm_batch {
         bool get = false;       // external: a lookup
         bool direct = false;    // external insert: the direct passes (else the component path)
         bool merge = false;     // external insert: the merge before them (tables without tombstones)
+        bool tombs = false;     // external insert: the table may hold tombstones then (queue_fill)
         double load = 0.0;      // external: the load it can reach (tuned tile width)
         uint32_t op = 0;        // external: the op
         fm::Shape shape = fm::SHAPE_GENERIC;
@@ -1513,6 +1539,15 @@ int queue_fill(fm_batch* b) {
                 break;
             }
     }
+    // what the host knows of each table's history when an insert runs
+    std::vector<char> tombs(b->tables.size()), before(b->ops.size());
+    for (size_t i = 0; i < b->tables.size(); i++) tombs[i] = b->tables[i]->tombs.load();
+    for (size_t i = 0; i < b->ops.size(); i++) {
+        before[i] = tombs[b->table_of[i]];
+        if (b->ops[i].kind == FM_OP_REMOVE && b->ops[i].n) tombs[b->table_of[i]] = 1;
+    }
+    for (auto& st : b->qsteps)
+        if (st.external) st.tombs = before[st.op];
     auto* q = reinterpret_cast<fm::QOp*>(b->h_desc + b->q_ops_off);
     for (size_t i = 0; i < b->ops.size(); i++) {
         const fm_op& o = b->ops[i];
@@ -1637,10 +1672,14 @@ int queue_enqueue(fm_batch* b, cudaStream_t s, bool adaptive) {
                 continue;
             }
             e = fm::launch_grp_ins(st.shape, dg + st.ext, 1, h.n, fm::GRP_BEGIN, 0, 0, s);
-            if (e == cudaSuccess && st.merge && h.sc.carry)
+            if (e == cudaSuccess && st.merge && !st.tombs && h.sc.carry)
                 e = fm::launch_ins_merge_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, s);
             if (e == cudaSuccess && st.direct) {
-                e = fm::launch_ins_direct_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, st.load, s);
+                // a graph may be replayed on another history than the
+                // capture's, which the device sees
+                fm::DxHow how = adaptive ? fm::DX_ALONE : fm::DX_EITHER;
+                if (st.tombs || !clean_passes_pay(b->ops[st.op].table, st.load, h.n)) how = fm::DX_GENERAL;
+                e = fm::launch_ins_direct_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, st.load, how, s);
                 if (e == cudaSuccess)
                     e = fm::launch_ins_comp(h.t, st.shape, h.keys, h.vals, fm::CMP_N0_CTL, 1, h.n, h.sc, h.ctl, s);
             } else if (e == cudaSuccess) {
@@ -2255,24 +2294,17 @@ int fm_batch_run(fm_batch* b, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     // tables must not have host-side work in flight on their own streams
     for (fm_table* t : b->tables) cudaStreamSynchronize(t->stream);
+    int rc = b->qmode ? queue_fill(b) : batch_fill(b);
+    if (!rc && b->exec && b->gens != scratch_gens(b)) rc = recapture(b);
+    if (rc) return rc;
     batch_note_history(b);
-    int rc;
     if (b->exec) {
-        rc = b->qmode ? queue_fill(b) : batch_fill(b);
-        if (!rc && b->gens != scratch_gens(b)) rc = recapture(b);
-        if (rc) return rc;
         cudaError_t e = cudaGraphLaunch(b->exec, s);
         if (e != cudaSuccess) return cuda_fail(FM_ERR_KERNEL_LAUNCH, "graph launch", e);
         fm::count_launches((unsigned)b->launches_per_run);
     } else {
         TimerScope ts(b->tables.size() == 1 ? b->tables[0] : nullptr);
-        if (b->qmode) {
-            rc = queue_fill(b);
-            if (!rc) rc = queue_enqueue(b, s, true);
-        } else {
-            rc = batch_fill(b);
-            if (!rc) rc = batch_enqueue(b, s, true);
-        }
+        rc = b->qmode ? queue_enqueue(b, s, true) : batch_enqueue(b, s, true);
         if (rc) return rc;
     }
     b->last_stream = s;

@@ -2247,9 +2247,10 @@ __device__ __forceinline__ void dx_let_next() {
 // key is stored twice, an op whose key is stored before the call stays an
 // update whatever the others do, and updates move nothing, so they are told
 // apart in the find pass and written before the exec pass (the last op on
-// each key), and only new keys go through the components.
-__device__ __forceinline__ bool dx_clean(const TableView& t, const Ctl* ctl) {
-    return t.mask >= 7 && t.mask < (uint64_t)DIST_MASK && *(volatile const uint32_t*)&ctl->tomb_claimed == 0u;
+// each key), and only new keys go through the components.  (DX_GENERAL: the
+// host has chosen the passes for any table.)
+__device__ __forceinline__ bool dx_clean(const TableView& t, const Ctl* ctl, uint32_t how) {
+    return how != DX_GENERAL && t.mask >= 7 && t.mask < (uint64_t)DIST_MASK && *(volatile const uint32_t*)&ctl->tomb_claimed == 0u;
 }
 
 // First free slot at or after unwrapped position a, looking at no more than
@@ -2303,10 +2304,10 @@ __device__ __forceinline__ uint64_t dx_next_free(const TableView& t, uint64_t a,
 
 template <int KB>
 __global__ void __launch_bounds__(RBLOCK) k_dx_find(TableView t, const uint8_t* __restrict__ keys, uint32_t n0_arg,
-                                                    OpScratch sc, Ctl* ctl) {
+                                                    uint32_t how, OpScratch sc, Ctl* ctl) {
     dx_let_next();
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
-    const bool clean = dx_clean(t, ctl);
+    const bool clean = dx_clean(t, ctl, how);
     bool no_free = false;
     const uint32_t iters = grid_iters(n0);
     for (uint32_t it = 0; it < iters; it++) {  // warp-uniform trip count
@@ -2346,12 +2347,12 @@ __global__ void __launch_bounds__(RBLOCK) k_dx_find(TableView t, const uint8_t* 
 
 template <int VB>
 __global__ void __launch_bounds__(RBLOCK) k_dx_flow(TableView t, const uint8_t* __restrict__ vals, uint32_t n0_arg,
-                                                    OpScratch sc, Ctl* ctl) {
+                                                    uint32_t how, OpScratch sc, Ctl* ctl) {
     dx_wait_prev();
     dx_let_next();
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
     const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;  // every op goes to the component path, later
-    const bool clean = dx_clean(t, ctl);
+    const bool clean = dx_clean(t, ctl, how);
     const uint32_t iters = grid_iters(n0);
     for (uint32_t it = 0; it < iters; it++) {  // warp-uniform trip count
         const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x + it * gridDim.x * blockDim.x;
@@ -2655,17 +2656,17 @@ constexpr int DC_THREADS = 128;
 template <int KB, int VB>
 __global__ void __launch_bounds__(DC_THREADS, FM_DC_BLOCKS) k_dx_exec_clean(TableView t, const uint8_t* __restrict__ keys,
                                                                  const uint8_t* __restrict__ vals, uint32_t n0_arg,
-                                                                 uint32_t opw, bool alone, OpScratch sc, Ctl* ctl) {
+                                                                 uint32_t opw, uint32_t how, OpScratch sc, Ctl* ctl) {
     constexpr uint32_t FULL = 0xFFFFFFFFu, OWN = 0x2000u;  // list: lane << 8 | bit, OWN: the op's own entry
     constexpr uint32_t BM = FM_DC_BATCH;
     __shared__ uint16_t s_list[DC_THREADS / 32][32 * (DX_LCH + 1) + 1];
     __shared__ uint32_t s_tmp[DC_THREADS / 32];
     dx_wait_prev();
     dx_let_next();
-    const bool clean = dx_clean(t, ctl);  // block-uniform
-    // alone: k_dx_exec is not launched beside it.  Tombstones that the host
+    const bool clean = dx_clean(t, ctl, how);  // block-uniform
+    // DX_ALONE: k_dx_exec is not launched beside it.  Tombstones that the host
     // did not know of then send every op to the component path.
-    if (!clean && !alone) return;
+    if (!clean && how != DX_ALONE) return;
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
     const bool to_pend = n0_arg == CMP_N0_CTL;  // as k_dx_exec
     const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0 || !clean;
@@ -2761,7 +2762,7 @@ __global__ void __launch_bounds__(DC_THREADS, FM_DC_BLOCKS) k_dx_exec_clean(Tabl
 template <int KB, int VB>
 __global__ void __launch_bounds__(DX_THREADS, DX_BLOCKS) k_dx_exec(TableView t, const uint8_t* __restrict__ keys,
                                                            const uint8_t* __restrict__ vals, uint32_t n0_arg,
-                                                           OpScratch sc, Ctl* ctl) {
+                                                           uint32_t how, OpScratch sc, Ctl* ctl) {
     __shared__ DxLaneSmem s_lane;
     __shared__ uint32_t s_tmp[DX_THREADS / 32];
     dx_wait_prev();
@@ -2773,7 +2774,7 @@ __global__ void __launch_bounds__(DX_THREADS, DX_BLOCKS) k_dx_exec(TableView t, 
     const bool to_pend = n0_arg == CMP_N0_CTL;
     const bool serial = *(volatile uint32_t*)&ctl->serial[0] != 0;
     const bool lanes_ok = t.mask >= 7 && t.mask < (uint64_t)DIST_MASK;
-    if (dx_clean(t, ctl)) return;  // block-uniform: k_dx_exec_clean
+    if (dx_clean(t, ctl, how)) return;  // block-uniform: k_dx_exec_clean
     ExecAcc a;
     // ops taken 32 at a time per warp, after the first from a counter
     // (Ctl::exec_next, zero at the start of the call): the grid is the resident
@@ -3033,6 +3034,7 @@ __device__ __noinline__ uint32_t dx_gather_q(const TableView& t, uint32_t j, uin
 // 7K walks that do not fit the bits.
 constexpr uint32_t CF_SLOTS = 512;  // slots of a component run this way
 constexpr uint32_t CF_TAKE = 4;     // entries a warp takes at a time
+static_assert(CLEAN_MIN_SLOTS >= 2 * CF_SLOTS, "offsets of a component's homes");
 struct __align__(16) CfSmem {  // moved in 16- and 8-byte pieces
     uint32_t flags[CF_SLOTS];
     uint16_t c[CF_SLOTS];    // ops that start at a slot (0/1), then c, then the destinations in order
@@ -3075,7 +3077,7 @@ __device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restric
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t m32 = (uint32_t)t.mask;
-    if (t.mask < 4 * CF_SLOTS) return false;
+    if (t.mask + 1 < CLEAN_MIN_SLOTS) return false;  // the homes' offsets below would run into one another
     // the ops' homes from CF_SLOTS before F on
     const uint32_t org = (uint32_t)F - CF_SLOTS;
     uint32_t op[2], q[2];
@@ -3139,7 +3141,10 @@ __device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restric
         reinterpret_cast<uint2*>(s.src + len)[lane] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
         len += 128;
     }
-    if (top - low + al >= len) return false;  // never expected: every op's free slot is one of the n
+    // With repeats the flow pass counted more ops than there are keys, and a
+    // home may lie beyond the n free slots, or its ops' way to theirs beyond
+    // what was read (end == 0 below): not for this pass.
+    if (top - low + al >= len) return false;
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < 2; u++)
@@ -3181,7 +3186,7 @@ __device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restric
         s.c[w + lane] = (uint16_t)cl;
     }
     __syncwarp();
-    if (end == 0) return false;  // never expected
+    if (end == 0) return false;
     // where every entry goes
     for (uint32_t x = lane; x < end; x += 32) {
         const uint32_t f = s.flags[x];
@@ -3250,24 +3255,26 @@ __device__ __noinline__ bool cf_run(const TableView& t, const uint8_t* __restric
 // The component pass: on a table without tombstones, the entries the exec
 // pass listed, a warp each (cf_run).  An entry that spans too many slots is
 // passed on: its ops to pend[0], offset and count to op_pt (Ctl::nbig of
-// them), for the warp pass.  Bound by the latency of each entry's chain of
+// them), for the warp pass, or where there is none to pend[1], for the
+// component path.  Bound by the latency of each entry's chain of
 // dependent reads (its lists, metadata, records), so it takes the registers
 // that let four blocks stay on an SM (two in the warp pass).
 template <int KB, int VB>
 __global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t* __restrict__ keys,
-                                                     const uint8_t* __restrict__ vals, uint32_t n0_arg, OpScratch sc,
-                                                     Ctl* ctl, Ctl* host) {
+                                                     const uint8_t* __restrict__ vals, uint32_t n0_arg, uint32_t how,
+                                                     OpScratch sc, Ctl* ctl, Ctl* host) {
     __shared__ CfSmem s_cf[RBLOCK / 32];
     __shared__ uint32_t s_ops[RBLOCK / 32][CF_TAKE][DX_GATHER];
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     dx_wait_prev();
     dx_let_next();
     const uint32_t n = *(volatile const uint32_t*)&ctl->nlong[0];
-    if (n == 0 || !dx_clean(t, ctl)) {  // block-uniform
+    if (n == 0 || !dx_clean(t, ctl, how)) {  // block-uniform
         publish_call(ctl, host);
         return;
     }
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
+    const bool to_pend = how == DX_ALONE && n0_arg == CMP_N0_CTL;  // no warp pass behind this one
     const Tile<32> tl;
     const uint32_t wi = threadIdx.x >> 5;
     ExecAcc a;
@@ -3297,13 +3304,18 @@ __global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t*
             if (!cf_run<KB, VB>(t, keys, vals, ops, g, F, sc, s_cf[wi], a)) {
                 uint32_t at = 0;
                 if (tl.lane == 0) {
-                    at = atomicAdd(&ctl->big_ops, g);
-                    const uint32_t k = atomicAdd(&ctl->nbig, 1u);
-                    sc.op_pt[(uint64_t)k * PT_MAX + 1] = at;
-                    sc.op_pt[(uint64_t)k * PT_MAX + 2] = g;
+                    if (to_pend) {
+                        at = atomicAdd(&ctl->npend[1], g);
+                    } else {
+                        at = atomicAdd(&ctl->big_ops, g);
+                        const uint32_t k = atomicAdd(&ctl->nbig, 1u);
+                        sc.op_pt[(uint64_t)k * PT_MAX + 1] = at;
+                        sc.op_pt[(uint64_t)k * PT_MAX + 2] = g;
+                    }
                 }
                 at = tl.shfl(at, 0);
-                for (uint32_t x = tl.lane; x < g; x += 32) sc.pend[0][at + x] = ops[x];
+                uint32_t* left = to_pend ? sc.pend[1] : sc.pend[0];
+                for (uint32_t x = tl.lane; x < g; x += 32) left[at + x] = ops[x];
             }
             tl.sync();
         }
@@ -3320,13 +3332,13 @@ __global__ void __launch_bounds__(RBLOCK, 4) k_dx_cf(TableView t, const uint8_t*
 template <int KB, int VB, int T>
 __global__ void __launch_bounds__(RBLOCK, FM_P4_MIN_BLOCKS) k_dx_warp(TableView t, const uint8_t* __restrict__ keys,
                                                                       const uint8_t* __restrict__ vals, uint32_t n0_arg,
-                                                                      OpScratch sc, Ctl* ctl) {
+                                                                      uint32_t how, OpScratch sc, Ctl* ctl) {
     constexpr int NT = RBLOCK / T;
     __shared__ P4Chain<T> s_chain[NT];
     __shared__ uint32_t s_ops[NT][DX_GATHER];
     __shared__ uint32_t s_tmp[RBLOCK / 32];
     dx_wait_prev();
-    const bool fresh = dx_clean(t, ctl);  // then: the entries the component pass left
+    const bool fresh = dx_clean(t, ctl, how);  // then: the entries the component pass left
     const uint32_t n = *(volatile const uint32_t*)(fresh ? &ctl->nbig : &ctl->nlong[0]);
     if (n == 0) return;  // block-uniform
     const uint32_t n0 = cmp_n0(n0_arg, ctl);
@@ -4191,53 +4203,59 @@ constexpr Shape sh_of() {
 
 template <int KB, int VB>
 void warp_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                const OpScratch& sc, Ctl* ctl, float load, bool pdl, cudaStream_t s) {
+                const OpScratch& sc, Ctl* ctl, float load, bool pdl, DxHow how, cudaStream_t s) {
     if constexpr (KB != 0 && VB != 0) {
         const int tw = tuned_ins_cfg(sh_of<KB, VB>(), (double)load).tile;
         const unsigned gwt = grid_for((uint64_t)nmax * tw, FM_P4_MIN_BLOCKS);
-        if (tw == 8) launch_dependent(k_dx_warp<KB, VB, 8>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
-        else if (tw == 16) launch_dependent(k_dx_warp<KB, VB, 16>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
-        else launch_dependent(k_dx_warp<KB, VB, 32>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, sc, ctl);
+        const uint32_t h = how;
+        if (tw == 8) launch_dependent(k_dx_warp<KB, VB, 8>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, h, sc, ctl);
+        else if (tw == 16) launch_dependent(k_dx_warp<KB, VB, 16>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, h, sc, ctl);
+        else launch_dependent(k_dx_warp<KB, VB, 32>, gwt, RBLOCK, s, pdl, t, keys, vals, n0, h, sc, ctl);
     }
 }
 
 template <int KB, int VB>
 void direct_shape(const TableView& t, const uint8_t* keys, const uint8_t* vals, uint32_t n0, uint32_t nmax,
-                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, bool clean, Ctl* host, cudaStream_t s) {
+                  const OpScratch& sc, Ctl* ctl, float load, bool pdl_ok, DxHow how, Ctl* host, cudaStream_t s) {
     if constexpr (KB == 0 || VB == 0) {
         return;
     } else {
+        const bool pdl = pdl_ok && FM_DX_PDL != 0 && !kt_active();
         const unsigned g = grid_for(nmax, 8);
-        // with per-kernel timing on, events sit between the kernels, so they
-        // run as plain launches
-        const bool pdl = pdl_ok && FM_DX_PDL && !kt_active();
+        const uint32_t h = how;
         {
             KtScope kt(KC_INS_FIND, s);
-            k_dx_find<KB><<<g, RBLOCK, 0, s>>>(t, keys, n0, sc, ctl);
+            // waits for the earlier work on the stream in full (it reads the
+            // table and the registrations)
+            launch_dependent(k_dx_find<KB>, g, RBLOCK, s, false, t, keys, n0, h, sc, ctl);
         }
         {
             KtScope kt(KC_INS_WALK, s);
-            launch_dependent(k_dx_flow<VB>, g, RBLOCK, s, pdl, t, vals, n0, sc, ctl);
+            launch_dependent(k_dx_flow<VB>, g, RBLOCK, s, pdl, t, vals, n0, h, sc, ctl);
         }
         {
             KtScope kt(KC_INS_EXEC, s);
-            const unsigned ge = grid_for(nmax, DX_BLOCKS);  // the resident blocks at most
-            const uint64_t warps = (uint64_t)num_sms() * FM_DC_BLOCKS * (DC_THREADS / 32);  // resident
-            const uint32_t opw = nmax <= warps * 4 ? 4 : (nmax <= warps * 8 ? 8 : (nmax <= warps * 16 ? 16 : 32));
-            const uint64_t per_block = (uint64_t)opw * (DC_THREADS / 32);
-            const unsigned gx = (unsigned)std::min<uint64_t>((nmax + per_block - 1) / per_block, (uint64_t)num_sms() * 64);
-            launch_dependent(k_dx_exec_clean<KB, VB>, gx,
-                             DC_THREADS, s, pdl, t, keys, vals, n0, opw, clean, sc, ctl);
-            if (!clean)
-                launch_dependent(k_dx_exec<KB, VB>, ge, DX_THREADS, s, pdl, t, keys, vals, n0, sc, ctl);
+            if (how != DX_GENERAL) {
+                const uint64_t warps = (uint64_t)num_sms() * FM_DC_BLOCKS * (DC_THREADS / 32);  // resident
+                const uint32_t opw = nmax <= warps * 4 ? 4 : (nmax <= warps * 8 ? 8 : (nmax <= warps * 16 ? 16 : 32));
+                const uint64_t per_block = (uint64_t)opw * (DC_THREADS / 32);
+                const unsigned gx =
+                    (unsigned)std::min<uint64_t>((nmax + per_block - 1) / per_block, (uint64_t)num_sms() * 64);
+                launch_dependent(k_dx_exec_clean<KB, VB>, gx, DC_THREADS, s, pdl, t, keys, vals, n0, opw, h, sc, ctl);
+            }
+            if (how != DX_ALONE) {
+                const unsigned ge = grid_for(nmax, DX_BLOCKS);  // the resident blocks at most
+                launch_dependent(k_dx_exec<KB, VB>, ge, DX_THREADS, s, pdl, t, keys, vals, n0, h, sc, ctl);
+            }
         }
         {
             KtScope kt(KC_INS_LONG, s);
-            launch_dependent(k_dx_cf<KB, VB>, grid_for((uint64_t)nmax * 32, 4), RBLOCK, s, pdl, t, keys, vals, n0, sc,
-                             ctl, clean ? host : nullptr);
-            if (!clean) warp_shape<KB, VB>(t, keys, vals, n0, nmax, sc, ctl, load, pdl, s);
+            if (how != DX_GENERAL)
+                launch_dependent(k_dx_cf<KB, VB>, grid_for((uint64_t)nmax * 32, 4), RBLOCK, s, pdl, t, keys, vals, n0, h,
+                                 sc, ctl, how == DX_ALONE ? host : nullptr);
+            if (how != DX_ALONE) warp_shape<KB, VB>(t, keys, vals, n0, nmax, sc, ctl, load, pdl, how, s);
         }
-        count_launches(clean ? 4 : 6);
+        count_launches(how == DX_EITHER ? 6 : 4);
     }
 }
 
@@ -4263,9 +4281,9 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 }
 
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, bool clean, Ctl* host, cudaStream_t s) {
+                              const OpScratch& sc, Ctl* ctl, double load, DxHow how, Ctl* host, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, clean, host, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, true, how, host, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     return cudaGetLastError();
@@ -4274,7 +4292,7 @@ cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys,
 cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                                    const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
     KtScope kt(KC_INS_LONG, s);
-#define FM_CALL(K, V) warp_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, false, s)
+#define FM_CALL(K, V) warp_shape<K, V>(t, keys, vals, n0, n0, sc, ctl, (float)load, false, DX_ALONE, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     count_launches(1);
@@ -4282,9 +4300,9 @@ cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* 
 }
 
 cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
-                                  uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s) {
+                                  uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, DxHow how, cudaStream_t s) {
     if (sh == SHAPE_GENERIC || !sc.comp) return cudaErrorInvalidValue;
-#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, false, nullptr, s)
+#define FM_CALL(K, V) direct_shape<K, V>(t, keys, vals, CMP_N0_CTL, nmax, sc, ctl, (float)load, false, how, nullptr, s)
     FM_SHAPE_SWITCH(sh, FM_CALL)
 #undef FM_CALL
     return cudaGetLastError();

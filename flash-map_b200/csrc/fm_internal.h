@@ -133,14 +133,19 @@ cudaError_t launch_ins_rounds(const TableView& t, Shape sh, const uint8_t* keys,
 // ran and every op is left to launch_ins_comp at round 0; otherwise
 // Ctl::npend[1] ops (components too large for a warp) are left in pend[1]
 // for launch_ins_comp at round 1.
-// `clean`: the host knows that the table holds no tombstones, and the passes
-// for other tables are not launched (else both, and the device tells; should
-// it hold some after all, serial[0] leaves every op as above); then `host`
-// (pinned) takes the control block at the call's end, which is left
-// reset unless ctl_left, and what the component pass left (nbig) is left to
-// launch_ins_direct_warp.
+// `how` names the passes that are launched:
+//   DX_GENERAL  those for any table (find, flow, exec, warp)
+//   DX_ALONE    those for tables without tombstones, which the host takes the
+//               table for (find, flow, exec_clean, cf; should it hold some
+//               after all, serial[0] leaves every op as above).  `host`
+//               (pinned) takes the control block at the call's end, which is
+//               left reset unless ctl_left, and what the component pass left
+//               (nbig) is left to launch_ins_direct_warp
+//   DX_EITHER   both, and the device tells (graphs replayed on tables whose
+//               history is known only then)
+enum DxHow : uint32_t { DX_EITHER = 0, DX_GENERAL, DX_ALONE };
 cudaError_t launch_ins_direct(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
-                              const OpScratch& sc, Ctl* ctl, double load, bool clean, Ctl* host, cudaStream_t s);
+                              const OpScratch& sc, Ctl* ctl, double load, DxHow how, Ctl* host, cudaStream_t s);
 // The warp pass alone, for what the component pass left (Ctl::nbig).
 cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals, uint32_t n0,
                                    const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s);
@@ -148,8 +153,13 @@ cudaError_t launch_ins_direct_warp(const TableView& t, Shape sh, const uint8_t* 
 // its precheck; nmax bounds it and sizes the grids) and no host step after
 // them: a call that found no free slot lists every op in pend[1], so
 // launch_ins_comp at round 1 with CMP_N0_CTL completes the call either way.
+// With DX_ALONE the component pass leaves the entries that are too long for it
+// there too.
 cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* keys, const uint8_t* vals,
-                                  uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, cudaStream_t s);
+                                  uint32_t nmax, const OpScratch& sc, Ctl* ctl, double load, DxHow how,
+                                  cudaStream_t s);
+// Smallest table of the component pass (twice the slots it takes in at once).
+constexpr uint64_t CLEAN_MIN_SLOTS = 1024;
 // A whole insert call of n0 ops merged into a table without tombstones
 // (compile-time record shapes, MG_MIN_SLOTS to 2^28 slots, OpScratch::carry).
 // On return (stream-ordered) Ctl::serial[0] set means that no record has
