@@ -361,20 +361,39 @@ bool note_history(fm_table* t) {
     return h != 0;
 }
 
-// Whether an insert of n ops runs as a merge: a table without tombstones, and
-// a call large enough beside the table that passes over all its slots cost
-// less than per-op work, and a load below FM_DIRECT_LOAD after it (beyond,
-// the runs are long and carry more ops than the merge keeps).  Per call of
-// account pairs into 2^21 slots, direct against merged: 1/41 of the table
-// 64-108 against 130-150 us, 1/20 84-166 against 134-173 us (from empty to
-// load 0.8); 1/4 (4M u64 keys into 2^24) 8.4 against 1.3 ms.
+// Whether an insert of n ops that may take the table to `reach` of its slots
+// pays as a merge: the merge's passes over all slots cost about as much
+// whatever the load, a direct call's time grows with the length of its walks.
+// In us, direct against merged, where n / (1 - reach)^1.5 is about the line of
+// 10.8 capacity^0.72 and on either side of it (call and wait):
+//   u64 pairs      2^13 slots, 1/4 of them: empty 58 / 71, load 0.4 87 / 83, 0.6 598 / 142
+//                  2^20 slots, 1/16: empty 65 / 104, load 0.6 117 / 118, 0.85 1318 / 304
+//                  2^24 slots, 1/16: empty 475 / 540, load 0.4 642 / 597; 1/8: empty 1098 / 692
+//   account pairs  2^16 slots, 1/8: empty 59 / 79, load 0.6 109 / 103
+//                  2^20 slots, 1/16: empty 74 / 110, load 0.6 139 / 140, 0.85 2516 / 406
+//                  2^20 slots, 1/4: empty 204 / 146; 2^24 slots, 1/16: load 0.4 707 / 708
+// Over 322 such calls (u64, 32/32 and account pairs, 2^13 to 2^24 slots, 1/16
+// to 1/2 of them, loads 0 to 0.9) the rule's choice took 1.002 times the
+// better one's time on average and 1.16 at most; merging every one of them
+// 1.08 and 1.59.
+// From FM_DIRECT_LOAD on the runs carry more ops than the merge keeps.
 #ifndef FM_MERGE_RATIO
 #define FM_MERGE_RATIO 16
 #endif
+double merge_gain(uint64_t cap, double reach, uint64_t n) {
+    const double gap = std::max(1.0 - reach, 1e-3);
+    return (double)n / (gap * std::sqrt(gap)) / (10.8 * std::pow((double)cap, 0.72));
+}
+
+// Whether an insert of n ops runs as a merge: a table without tombstones, a
+// call large enough beside the table.  The one-launch form for small tables
+// pays from 1/16 of the slots at every load (256 account pairs into 2^12 slots:
+// empty 38 against 44 us, load 0.85 76 against 231).
 bool merge_wanted(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n) {
+    const double reach = (double)(len + n) / (double)t->cap;
     return sh != fm::SHAPE_GENERIC && !t->tombs.load() && t->cap >= fm::MG_MIN_SLOTS &&
            t->mask < (uint64_t)fm::DIST_MASK && n <= fm::MG_MAX_OPS && n * FM_MERGE_RATIO >= t->cap &&
-           (double)(len + n) < FM_DIRECT_LOAD * (double)t->cap;
+           reach < FM_DIRECT_LOAD && (t->cap <= fm::MG_SMALL_SLOTS || merge_gain(t->cap, reach, n) >= 1.0);
 }
 
 // Whether a direct insert of n ops into a table without tombstones runs on
@@ -1420,7 +1439,7 @@ struct fm_batch {
         bool remove = false;    // external: a remove
         bool get = false;       // external: a lookup
         bool direct = false;    // external insert: the direct passes (else the component path)
-        bool merge = false;     // external insert: the merge before them (tables without tombstones)
+        double merge = 0.0;     // external insert: what a merge before them gains (merge_gain; 0: none)
         bool tombs = false;     // external insert: the table may hold tombstones then (queue_fill)
         double load = 0.0;      // external: the load it can reach (tuned tile width)
         uint32_t op = 0;        // external: the op
@@ -1534,7 +1553,7 @@ int queue_fill(fm_batch* b) {
         if (rc) return rc;
         // (a table whose plan has a merge; its address does not change)
         for (const auto& st : b->qsteps)
-            if (st.merge && b->table_of[st.op] == i) {
+            if (st.merge > 0.0 && b->table_of[st.op] == i) {
                 ensure_carry(b->tables[i]);
                 break;
             }
@@ -1672,7 +1691,10 @@ int queue_enqueue(fm_batch* b, cudaStream_t s, bool adaptive) {
                 continue;
             }
             e = fm::launch_grp_ins(st.shape, dg + st.ext, 1, h.n, fm::GRP_BEGIN, 0, 0, s);
-            if (e == cudaSuccess && st.merge && !st.tombs && h.sc.carry)
+            // an eager run is bound by its launches, and the merge is eleven
+            // more (32 inserts of 2000 pairs into tables of 2^14 slots, all merged:
+            // 2.8 ms, none 1.8)
+            if (e == cudaSuccess && st.merge > (adaptive ? 2.0 : 0.0) && !st.tombs && h.sc.carry)
                 e = fm::launch_ins_merge_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, s);
             if (e == cudaSuccess && st.direct) {
                 // a graph may be replayed on another history than the
@@ -1731,10 +1753,13 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
     // the merge's kernels see for themselves when they run)
     std::vector<char> tombs(b->tables.size());
     for (size_t i = 0; i < b->tables.size(); i++) tombs[i] = b->tables[i]->tombs.load();
-    auto merges = [&](const fm_op& o, uint32_t ti) {
+    auto merges = [&](const fm_op& o, uint32_t ti) -> double {  // (est: with the op's keys)
         const fm_table* t = o.table;
-        return !tombs[ti] && t->cap >= fm::MG_MIN_SLOTS && t->mask < (uint64_t)fm::DIST_MASK && o.n <= fm::MG_MAX_OPS &&
-               o.n * FM_MERGE_RATIO >= t->cap;
+        if (tombs[ti] || t->cap < fm::MG_MIN_SLOTS || t->mask >= (uint64_t)fm::DIST_MASK || o.n > fm::MG_MAX_OPS ||
+            o.n * FM_MERGE_RATIO < t->cap)
+            return 0.0;
+        const double gain = merge_gain(t->cap, est[ti] / (double)t->cap, o.n);
+        return gain >= 1.0 ? gain : 0.0;
     };
     if (b->qlanes) {
         // every op a device-driven step: a table's inserts and removes on its
@@ -1775,7 +1800,7 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
             st.remove = o.kind == FM_OP_REMOVE;
             if (o.kind == FM_OP_INSERT) est[ti] = std::min(est[ti] + (double)o.n, cap);
             st.direct = est[ti] < FM_DIRECT_LOAD * cap;
-            st.merge = o.kind == FM_OP_INSERT && st.direct && merges(o, ti);
+            st.merge = o.kind == FM_OP_INSERT && st.direct ? merges(o, ti) : 0.0;
             if (o.kind == FM_OP_REMOVE) tombs[ti] = 1;
             st.load = est[ti] / cap;
             st.ext = (uint32_t)b->qext_ops.size();
@@ -1853,7 +1878,7 @@ void queue_plan(fm_batch* b, const std::vector<uint32_t>& lane_of) {
                 fm_batch::QStep st;
                 st.external = true;
                 st.direct = est[ti] < FM_DIRECT_LOAD * cap;
-                st.merge = st.direct && merges(o, ti);
+                st.merge = st.direct ? merges(o, ti) : 0.0;
                 st.load = est[ti] / cap;
                 st.op = i;
                 st.shape = o.table->shape;

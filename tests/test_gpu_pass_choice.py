@@ -135,3 +135,29 @@ def test_batched_inserts(shape, bits, run, graph):
     want = [(o.bulk_remove(k) if kind == F.batch.REMOVE else o.bulk_insert(k, v), 0) for kind, k, v in queue]
     assert b.wait() == want
     _same(g, o)
+
+
+@pytest.mark.parametrize("shape", [(8, 8), (32, 128)])
+@pytest.mark.parametrize("bits,load,part,merged", [(13, 0.0, 4, False), (13, 0.6, 4, True), (16, 0.0, 16, False),
+                                                   (16, 0.0, 8, False), (16, 0.85, 16, True), (16, 0.5, 2, True),
+                                                   (20, 0.0, 16, False), (20, 0.85, 16, True), (20, 0.0, 2, True)])
+def test_merges_where_they_pay(shape, bits, load, part, merged):
+    """A merge is ten launches, a direct call four: large calls on either side of the line."""
+    ks, vs = shape
+    cap = 1 << bits
+    rng = np.random.default_rng(bits + part)
+    from flash_map import _native
+    import torch
+
+    g, o = gpu_map(cap, ks, vs), O.OracleMap(cap, ks, vs)
+    if load:
+        k, v = _records(rng, int(cap * load), ks), _records(rng, int(cap * load), vs)
+        assert g.bulk_insert(k, v) == o.bulk_insert(k, v)
+    n = cap // part
+    k, v = _records(rng, n, ks), _records(rng, n, vs)
+    dk, dv = torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda()
+    torch.cuda.synchronize()
+    before = _native.launch_count()
+    assert g.bulk_insert_device(dk, dv, n) == o.bulk_insert(k, v)
+    assert (_native.launch_count() - before >= 10) == merged
+    _same(g, o)
