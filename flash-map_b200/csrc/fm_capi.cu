@@ -237,7 +237,6 @@ struct fm_table {
     size_t sc_bytes = 0;
     uint8_t* sc_base = nullptr;
     uint64_t sc_gen = 0;          // counts the scratch's moves (captured graphs hold its addresses)
-    uint32_t* d_carry = nullptr;  // merging inserts' words (ensure_carry)
     bool ctl_reset = true;        // d_ctl's per-call fields are zero (under mu; batches clear it)
     uint8_t* d_in = nullptr;  // host-API staging for mutating calls (two pieces)
     size_t d_in_cap = 0;
@@ -280,30 +279,32 @@ struct TimerScope {
     ~TimerScope() { tl_timer = prev; }
 };
 
-// The merging inserts' words of a table, allocated once: captured graphs hold
-// their address, so they do not move when the scratch grows.  Without room
-// for them the calls run without the merge.
-void ensure_carry(fm_table* t) {
-    if (!t->d_carry && cudaMalloc((void**)&t->d_carry, fm::mg_bytes(t->mask)) != cudaSuccess) {
-        t->d_carry = nullptr;
-        cudaGetLastError();
-    }
-    t->sc.carry = t->d_carry;
-}
-
-int ensure_scratch(fm_table* t, uint64_t n) {
-    if (t->sc.cap_ops >= n) return FM_OK;
+// Scratch for calls of n ops, with `carry` the merging inserts' words too.  One
+// block: an allocation of its own for the words cost the first merging call
+// of every table 350 us (65,536 pairs into a fresh table of 2^18 slots 490 us
+// instead of 94).  Without room for the words the calls run without the merge.
+int ensure_scratch(fm_table* t, uint64_t n, bool carry = false) {
+    if (t->sc.cap_ops >= n && (!carry || t->sc.carry)) return FM_OK;
+    carry = carry || t->sc.carry;
     // pend[0], pend[1] (u32) | op_slot (u64) | op_word (u32) | op_flag (u8) | op_pt (PT_MAX u32) |
     // long_list (u32) per op, then the component buffer and the remove chunk summaries (per table)
     const uint64_t per_op = 4 + 4 + 8 + 4 + 1 + 4 * fm::PT_MAX + 4;
-    const uint64_t want = n + n / 4 + 1024;
-    const size_t bytes = (size_t)(want * per_op + 9 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
+    const uint64_t want = std::max(n + n / 4 + 1024, t->sc.cap_ops);
+    size_t bytes = (size_t)(want * per_op + 10 * 256 + fm::cmp_bytes(t->mask) + 4 * fm::rsum_words(t->mask));
+    const size_t words = carry ? fm::mg_bytes(t->mask) : 0;
     if (t->sc_base) cudaFree(t->sc_base);
     t->sc_base = nullptr;
     t->sc = OpScratch{};
     t->sc_gen += 1;
-    cudaError_t e = dev_alloc((void**)&t->sc_base, bytes);
+    cudaError_t e = dev_alloc((void**)&t->sc_base, bytes + words);
+    if (e != cudaSuccess && carry) {
+        cudaGetLastError();
+        t->sc_base = nullptr;
+        carry = false;
+        e = dev_alloc((void**)&t->sc_base, bytes);
+    }
     if (e != cudaSuccess) return cuda_fail(FM_ERR_GPU_ALLOC, "scratch allocation", e);
+    if (carry) bytes += words;
     uint8_t* p = t->sc_base;
     auto carve = [&](size_t b) {
         uint8_t* r = p;
@@ -319,7 +320,7 @@ int ensure_scratch(fm_table* t, uint64_t n) {
     t->sc.long_list = (uint32_t*)carve(want * 4);
     t->sc.comp = carve(fm::cmp_bytes(t->mask));
     t->sc.rsum = (uint32_t*)carve(4 * fm::rsum_words(t->mask));
-    t->sc.carry = t->d_carry;
+    if (carry) t->sc.carry = (uint32_t*)carve(words);
     t->sc.cap_ops = want;
     t->sc_bytes = bytes;
     // op_word doubles as the insert inflow bound: idle value 0xFFFFFFFF.
@@ -396,6 +397,23 @@ bool merge_wanted(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n) {
            reach < FM_DIRECT_LOAD && (t->cap <= fm::MG_SMALL_SLOTS || merge_gain(t->cap, reach, n) >= 1.0);
 }
 
+// Whether the scratch for an insert of n ops takes in the merge's words: when
+// it is allocated for this call anyway and the call merges, or is of a size
+// that will at a higher load and the words do not take the allocation out of
+// the driver's small ones (10 us; from one or two megabytes on 400 us, hardly
+// more for larger ones); of a scratch that is there, where the merge gains more
+// than the 400 us of allocating it again (2^20 slots, 1/16 of them: 43 us at a
+// gain of 3.5, 2.1 ms at 11).
+bool carry_pays(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n, bool merge) {
+    if (t->cap <= fm::MG_SMALL_SLOTS || sh == fm::SHAPE_GENERIC || t->tombs.load()) return false;
+    if (t->sc.cap_ops < n) {
+        constexpr uint64_t SMALL = 5ull << 18;
+        const uint64_t ops = n * 52;  // the per-op part
+        return merge || (n * FM_MERGE_RATIO >= t->cap && (ops >= SMALL || ops + fm::mg_bytes(t->mask) < SMALL));
+    }
+    return merge && merge_gain(t->cap, (double)(len + n) / (double)t->cap, n) >= 6.0;
+}
+
 // Whether a direct insert of n ops into a table without tombstones runs on
 // the passes for such tables.  They lose where the component pass leaves
 // entries of more than its 512 slots to the warp pass: that is a second wait,
@@ -441,9 +459,8 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
         }
         note_history(t);
     }
-    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK);
+    int rc = ensure_scratch(t, n < OP_CHUNK ? n : OP_CHUNK, insert && carry_pays(t, sh, t->len.load(), n, merge));
     if (rc) return rc;
-    if (merge && t->cap > fm::MG_SMALL_SLOTS) ensure_carry(t);
     fm::TableView v = t->view();
     for (uint64_t base = 0; base < n; base += OP_CHUNK) {
         const uint32_t m = (uint32_t)((n - base) < OP_CHUNK ? (n - base) : OP_CHUNK);
@@ -774,7 +791,6 @@ void fm_destroy(fm_table* t) {
     cudaFree(t->d_ctl);
     if (t->h_ctl) cudaFreeHost(t->h_ctl);
     if (t->sc_base) cudaFree(t->sc_base);
-    if (t->d_carry) cudaFree(t->d_carry);
     if (t->d_in) cudaFree(t->d_in);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
@@ -1549,14 +1565,10 @@ int queue_fill(fm_batch* b) {
         if (b->ops[i].kind != FM_OP_GET) need[b->table_of[i]] = std::max(need[b->table_of[i]], b->ops[i].n);
     for (size_t i = 0; i < b->tables.size(); i++) {
         if (!need[i]) continue;
-        int rc = ensure_scratch(b->tables[i], need[i]);
+        bool merges = false;
+        for (const auto& st : b->qsteps) merges = merges || (st.merge > 0.0 && b->table_of[st.op] == i);
+        int rc = ensure_scratch(b->tables[i], need[i], merges);
         if (rc) return rc;
-        // (a table whose plan has a merge; its address does not change)
-        for (const auto& st : b->qsteps)
-            if (st.merge > 0.0 && b->table_of[st.op] == i) {
-                ensure_carry(b->tables[i]);
-                break;
-            }
     }
     // what the host knows of each table's history when an insert runs
     std::vector<char> tombs(b->tables.size()), before(b->ops.size());
