@@ -188,8 +188,9 @@ __global__ void __launch_bounds__(BLOCK, 8) k_get_thread(TableView t, const uint
 
 // Run-time record sizes: a thread per query as k_get_thread, then the warp
 // moves its 32 values together in the widest pieces that the size and both
-// addresses allow.  One 8-lane tile per query (k_get<0, 0, 8>, which tables
-// of fewer than 8 slots keep) had an eighth of the probes in flight.
+// addresses allow.  One 8-lane tile per query (k_get<0, 0, 8>, which small
+// calls and tables of fewer than 8 slots keep) has an eighth of the probes in
+// flight.
 __global__ void __launch_bounds__(BLOCK) k_get_any(TableView t, const uint8_t* __restrict__ qkeys, uint64_t n,
                                                    uint8_t* __restrict__ out_vals, uint8_t* __restrict__ out_found) {
     const uint32_t lane = threadIdx.x & 31u, vsz = t.vsz;
@@ -285,13 +286,19 @@ void get_launch(const TableView& t, const uint8_t* q, uint64_t n, uint8_t* ov, u
     g_launches += 1;
 }
 
+constexpr uint64_t GET_TILE_QUERIES = 128;  // per SM: lookups of run-time sizes that tiles of 8 lanes run
+
 template <int KB, int VB>
 cudaError_t get_shape(const TableView& t, const uint8_t* q, uint64_t n, uint8_t* ov, uint8_t* of, GetCfg cfg,
                       cudaStream_t s) {
     int lanes = cfg.lanes;
     // one thread per query needs compile-time sizes and 8-slot windows
+    // run-time sizes: a thread per query once those fill the chip; few queries
+    // are bound by the latency of one, which a tile's lanes share (64/256-byte
+    // records, 2^20 slots, against a thread each: 1000 queries 0.63 of the time,
+    // 16,000 0.72, 32,000 1.14; 5/3 bytes 0.63, 0.75, 1.0)
     if constexpr (KB == 0) {
-        if (lanes == 1 && t.mask >= 7) {
+        if (lanes == 1 && t.mask >= 7 && n > (uint64_t)num_sms() * GET_TILE_QUERIES) {
             KtScope kt(KC_GET, s);
             k_get_any<<<grid_for(n, cfg.blocks_per_sm), BLOCK, 0, s>>>(t, q, n, ov, of);
             g_launches += 1;
