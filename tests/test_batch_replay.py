@@ -123,3 +123,38 @@ def test_replay_after_the_scratch_has_grown(by):
             for g, b in zip(tables, saved):
                 g.copy_from(b, q.stream)
             q.check(oracles())
+
+
+@pytest.mark.parametrize("what", ["fits", "hot key", "hot home"])
+def test_replay_on_another_history(what):
+    """A graph planned for tables without tombstones, with a merged insert (one that the merge takes, or leaves for its
+    hot key or hot home), replayed without a rollback: from the second run on the tables hold tombstones, and the third
+    finds them reused."""
+    import flash_map as F
+
+    cap = 1 << 14
+    rng = np.random.default_rng(len(what))
+    tables = [gpu_map(cap, ks, vs) for ks, vs in SHAPES]
+    ops = []
+    for g in tables:
+        k = _records(rng, 7000, g.key_size)
+        if what == "hot key":
+            k[rng.choice(7000, 60, replace=False)] = k[0]
+        elif what == "hot home":
+            k[rng.choice(7000, 60, replace=False), :4] = k[0, :4]
+        small, late = _records(rng, 300, g.key_size), _records(rng, 200, g.key_size)
+        small[:100] = k[:100]
+        ops += [(g, F.batch.INSERT, k, _records(rng, 7000, g.value_size)),
+                (g, F.batch.INSERT, small, _records(rng, 300, g.value_size)),
+                (g, F.batch.REMOVE, np.concatenate([k[::3], small[::2], _records(rng, 100, g.key_size)]), None),
+                (g, F.batch.INSERT, late, _records(rng, 200, g.value_size)),
+                (g, F.batch.REMOVE, np.concatenate([late[::2], k[1::5]]), None),
+                (g, F.batch.GET, np.concatenate([k, small, late]), None)]
+    q = Queue(tables, ops)
+    oracles = {g: O.OracleMap(cap, g.key_size, g.value_size) for g in tables}
+    for _ in range(4):
+        q.check(oracles)
+    for g in tables:  # and from cleared tables again
+        g.clear()
+        oracles[g].clear()
+    q.check(oracles)
