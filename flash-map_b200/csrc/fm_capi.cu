@@ -366,24 +366,28 @@ bool note_history(fm_table* t) {
 // pays as a merge: the merge's passes over all slots cost about as much
 // whatever the load, a direct call's time grows with the length of its walks.
 // In us, direct against merged, where n / (1 - reach)^1.5 is about the line of
-// 10.8 capacity^0.72 and on either side of it (call and wait):
+// 8 capacity^0.72 and on either side of it (call and wait):
 //   u64 pairs      2^13 slots, 1/4 of them: empty 58 / 71, load 0.4 87 / 83, 0.6 598 / 142
 //                  2^20 slots, 1/16: empty 65 / 104, load 0.6 117 / 118, 0.85 1318 / 304
 //                  2^24 slots, 1/16: empty 475 / 540, load 0.4 642 / 597; 1/8: empty 1098 / 692
 //   account pairs  2^16 slots, 1/8: empty 59 / 79, load 0.6 109 / 103
 //                  2^20 slots, 1/16: empty 74 / 110, load 0.6 139 / 140, 0.85 2516 / 406
 //                  2^20 slots, 1/4: empty 204 / 146; 2^24 slots, 1/16: load 0.4 707 / 708
-// Over 322 such calls (u64, 32/32 and account pairs, 2^13 to 2^24 slots, 1/16
-// to 1/2 of them, loads 0 to 0.9) the rule's choice took 1.002 times the
-// better one's time on average and 1.16 at most; merging every one of them
-// 1.08 and 1.59.
+// Over 170 such calls (u64 and account pairs, 2^13 to 2^22 slots, 1/16 to 1/2
+// of them, loads 0 to 0.75) the rule's choice took 1.005 times the better one's
+// time on average and 1.21 at most, merging every one of them 1.1 and 1.6.
+// Repeats of a key cost a direct call more: with a fifth of them 1.011 and
+// 1.35 (with 10.8 in place of 8, the best without repeats, 1.014).
 // From FM_DIRECT_LOAD on the runs carry more ops than the merge keeps.
 #ifndef FM_MERGE_RATIO
 #define FM_MERGE_RATIO 16
 #endif
+#ifndef FM_MERGE_LINE
+#define FM_MERGE_LINE 8.0
+#endif
 double merge_gain(uint64_t cap, double reach, uint64_t n) {
     const double gap = std::max(1.0 - reach, 1e-3);
-    return (double)n / (gap * std::sqrt(gap)) / (10.8 * std::pow((double)cap, 0.72));
+    return (double)n / (gap * std::sqrt(gap)) / (FM_MERGE_LINE * std::pow((double)cap, 0.72));
 }
 
 // Whether an insert of n ops runs as a merge: a table without tombstones, a
@@ -403,7 +407,7 @@ bool merge_wanted(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n) {
 // the driver's small ones (10 us; from one or two megabytes on 400 us, hardly
 // more for larger ones); of a scratch that is there, where the merge gains more
 // than the 400 us of allocating it again (2^20 slots, 1/16 of them: 43 us at a
-// gain of 3.5, 2.1 ms at 11).
+// gain of 4.7, 2.1 ms at 15).
 bool carry_pays(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n, bool merge) {
     if (t->cap <= fm::MG_SMALL_SLOTS || sh == fm::SHAPE_GENERIC || t->tombs.load()) return false;
     if (t->sc.cap_ops < n) {
@@ -411,7 +415,7 @@ bool carry_pays(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n, bool 
         const uint64_t ops = n * 52;  // the per-op part
         return merge || (n * FM_MERGE_RATIO >= t->cap && (ops >= SMALL || ops + fm::mg_bytes(t->mask) < SMALL));
     }
-    return merge && merge_gain(t->cap, (double)(len + n) / (double)t->cap, n) >= 6.0;
+    return merge && merge_gain(t->cap, (double)(len + n) / (double)t->cap, n) >= 8.0;
 }
 
 // Whether a direct insert of n ops into a table without tombstones runs on
@@ -1706,7 +1710,7 @@ int queue_enqueue(fm_batch* b, cudaStream_t s, bool adaptive) {
             // an eager run is bound by its launches, and the merge is eleven
             // more (32 inserts of 2000 pairs into tables of 2^14 slots, all merged:
             // 2.8 ms, none 1.8)
-            if (e == cudaSuccess && st.merge > (adaptive ? 2.0 : 0.0) && !st.tombs && h.sc.carry)
+            if (e == cudaSuccess && st.merge > (adaptive ? 2.7 : 0.0) && !st.tombs && h.sc.carry)
                 e = fm::launch_ins_merge_ctl(h.t, st.shape, h.keys, h.vals, h.n, h.sc, h.ctl, s);
             if (e == cudaSuccess && st.direct) {
                 // a graph may be replayed on another history than the

@@ -139,7 +139,7 @@ def test_batched_inserts(shape, bits, run, graph):
 
 @pytest.mark.parametrize("shape", [(8, 8), (32, 128)])
 @pytest.mark.parametrize("bits,load,part,merged", [(13, 0.0, 4, False), (13, 0.6, 4, True), (16, 0.0, 16, False),
-                                                   (16, 0.0, 8, False), (16, 0.85, 16, True), (16, 0.5, 2, True),
+                                                   (16, 0.0, 8, False), (16, 0.85, 16, True), (16, 0.4, 2, True),
                                                    (20, 0.0, 16, False), (20, 0.85, 16, True), (20, 0.0, 2, True)])
 def test_merges_where_they_pay(shape, bits, load, part, merged):
     """A merge is ten launches, a direct call four: large calls on either side of the line."""
