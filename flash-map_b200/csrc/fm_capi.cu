@@ -485,8 +485,10 @@ int run_rounds_inner(fm_table* t, bool insert, const uint8_t* d_k, const uint8_t
             // (lone ops at once, each group in index order); ops the kernels
             // leave (no EMPTY slot anywhere, groups too large) run in rounds
             // -- or, while no insert has claimed a tombstone, in one pass in
-            // any order (a table filled to its last slot stays with the rounds
-            // and their bounded passes: it has no EMPTY slot for a probe to end at)
+            // any order (a table counted as full stays with the rounds; once
+            // removes have run on it, it still has no EMPTY slot, and an
+            // absent key's probe ends only at an entry nearer its home, as the
+            // find pass's would)
             const bool any_order = !t->claimed.load() && t->mask < (uint64_t)fm::DIST_MASK &&
                                    t->len.load() - total < t->cap;
             e = any_order ? fm::launch_rem_take(v, sh, kk, m, t->d_ctl, t->h_ctl, s)

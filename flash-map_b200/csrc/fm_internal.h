@@ -161,7 +161,7 @@ cudaError_t launch_ins_direct_ctl(const TableView& t, Shape sh, const uint8_t* k
 // Smallest table of the component pass (twice the slots it takes in at once).
 constexpr uint64_t CLEAN_MIN_SLOTS = 1024;
 // A whole insert call of n0 ops merged into a table without tombstones
-// (compile-time record shapes, MG_MIN_SLOTS to 2^28 slots, OpScratch::carry).
+// (compile-time record shapes, MG_MIN_SLOTS to 2^27 slots, OpScratch::carry).
 // On return (stream-ordered) Ctl::serial[0] set means that no record has
 // moved: seg_min and seg_cnt are to be set idle and the call run by another
 // path; otherwise every op is done.  (A table that turns out to hold
@@ -373,15 +373,15 @@ cudaError_t launch_grp_pending_each(const GroupOp* ops, uint32_t nops, uint32_t 
 // calling thread (no events otherwise).
 enum KernelClass : int {
     KC_GET = 0,     // k_get_thread / k_get
-    KC_INS_FIND,    // k_dx_find / k_ins_p1: first free slot, registration
-    KC_INS_WALK,    // k_dx_flow / k_ins_p2: flows over the free slots
-    KC_INS_EXEC,    // k_dx_exec / k_ins_p3: thread-per-op execution
-    KC_INS_LONG,    // k_dx_warp / k_ins_p4: warp-per-op execution (long walks, components)
+    KC_INS_FIND,    // k_dx_find / k_ins_p1: first free slot, registration; k_mg_find, k_mg_resolve
+    KC_INS_WALK,    // k_dx_flow / k_ins_p2: flows over the free slots; k_mg_fn .. k_mg_rank
+    KC_INS_EXEC,    // k_dx_exec_clean, k_dx_exec / k_ins_p3: an op per thread; k_mg_new, k_mg_old, k_mg_small
+    KC_INS_LONG,    // k_dx_cf, k_dx_warp / k_ins_p4: an entry per warp (long walks, components); k_mg_move
     KC_INS_TAIL,    // k_ins_tail: remaining rounds in one block
     KC_INS_SERIAL,  // k_ins_serial
     KC_REM_MARK,    // k_rx_find / k_rem_p1
     KC_REM_CHECK,   // k_rem_p2
-    KC_REM_EXEC,    // k_rx_exec / k_rem_p3
+    KC_REM_EXEC,    // k_rx_take, k_rx_exec / k_rem_p3
     KC_REM_TAIL,    // k_rem_tail
     KC_COUNT_OCC,   // k_count
     KC_REM_GROUP,   // k_rx_warp: a warp per group of removes
