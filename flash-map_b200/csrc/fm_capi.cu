@@ -429,16 +429,21 @@ bool carry_pays(const fm_table* t, fm::Shape sh, uint64_t len, uint64_t n, bool 
 // 32/32 and account pairs, 2^13 to 2^23 slots, loads 0.80 to 0.94, 4 to 100,000
 // ops).  Account pairs into 2^20 slots: load 0.80, 1000 ops 79 against 120 us;
 // load 0.85, 256 ops 76 against 96, 10,000 ops 160 against 308; load 0.90, 256
-// ops 195 against 160, 10,000 ops 875 against 791.  The component pass needs
-// 1024 slots: of a smaller table it left every new key (64 to 256 slots: 62
-// against 36 us a call).
+// ops 195 against 160, 10,000 ops 875 against 791.  What the warp pass adds does
+// not grow with the call, what these passes save does: from 200,000 ops on they
+// are the quicker ones at every load (400,000 account pairs into 2^24 slots:
+// load 0.81 613 against 1055 us, 0.86 1256 against 1571, 0.93 7389 against
+// 7908), and the line rises from 20,000 ops on (100,000 u64 pairs into 2^24
+// slots: load 0.84 191 against 252, 0.86 404 against 313).  The component pass
+// needs 1024 slots: of a smaller table it left every new key (64 to 256 slots:
+// 62 against 36 us a call).
 #ifndef FM_CLEAN_WALK
 #define FM_CLEAN_WALK 450.0
 #endif
 bool clean_passes_pay(const fm_table* t, double reach, uint64_t n) {
-    const double gap = 1.0 - reach;
-    return t->cap >= fm::CLEAN_MIN_SLOTS && t->mask < (uint64_t)fm::DIST_MASK && gap > 0.0 &&
-           (double)n * std::exp(-FM_CLEAN_WALK * gap * gap) < 0.25;
+    if (t->cap < fm::CLEAN_MIN_SLOTS || t->mask >= (uint64_t)fm::DIST_MASK || reach >= 1.0) return false;
+    const double gap = 1.0 - reach, e = (double)n * std::exp(-FM_CLEAN_WALK * gap * gap);
+    return n >= 200000 || e < 0.25 * std::max(1.0, (double)n / 20000.0);
 }
 
 // The round driver shared by insert and remove.  Each pass launches two

@@ -24,7 +24,8 @@ def _same(g, o):
 @pytest.mark.parametrize("shape", [(8, 8), (32, 128)])
 @pytest.mark.parametrize("claim", [False, True])
 @pytest.mark.parametrize("bits,call", [(14, "insert 100"), (14, "insert 1300"), (12, "insert 300"), (12, "insert 20"),
-                                       (9, "insert 20"), (14, "remove 400"), (9, "remove 40")])
+                                       (9, "insert 20"), (14, "remove 400"), (9, "remove 40"), (14, "batch 100"),
+                                       (14, "batch 5000"), (11, "batch 40"), (9, "batch 20")])
 def test_call_after_a_clear_that_ran_ahead_of_a_batch(shape, claim, bits, call):
     import torch
 
@@ -57,7 +58,15 @@ def test_call_after_a_clear_that_ran_ahead_of_a_batch(shape, claim, bits, call):
     _same(g, o)
     kind, m = call.split()
     m = int(m)
-    if kind == "insert":
+    if kind == "batch":  # queued without a graph: its passes are chosen when it runs
+        q, w = _records(rng, m, ks), _records(rng, m, vs)
+        q[: m // 3] = k[: m // 3]
+        dq, dw = torch.from_numpy(q).cuda(), torch.from_numpy(w).cuda()
+        torch.cuda.synchronize()
+        b2 = F.FlashMapBatch([F.BatchOp(F.batch.INSERT, g, m, dq, dw)])
+        b2.run(s)
+        assert b2.wait() == [(o.bulk_insert(q, w), 0)]
+    elif kind == "insert":
         q = np.concatenate([k[: m // 3], gone[: m // 3], _records(rng, m - m // 3 * 2, ks)])
         q = q[rng.permutation(len(q))]
         w = _records(rng, len(q), vs)

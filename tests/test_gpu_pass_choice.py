@@ -161,3 +161,18 @@ def test_merges_where_they_pay(shape, bits, load, part, merged):
     assert g.bulk_insert_device(dk, dv, n) == o.bulk_insert(k, v)
     assert (_native.launch_count() - before >= 10) == merged
     _same(g, o)
+
+
+def test_large_calls_at_high_load():
+    """200,000 ops and more keep to the passes for tables without tombstones at every load, entries that are too long
+    for the component pass among them."""
+    cap = 1 << 22
+    rng = np.random.default_rng(11)
+    g, o = gpu_map(cap, 8, 8), O.OracleMap(cap, 8, 8)
+    k = _records(rng, int(cap * 0.85), 8)
+    assert g.bulk_insert(k, k) == o.bulk_insert(k, k)
+    for n in (200_000, 199_999):
+        k = _records(rng, n, 8)
+        k[::50] = k[7]  # one key many times
+        _insert(g, o, k, rng)
+    _same(g, o)
