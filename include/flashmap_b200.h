@@ -200,7 +200,8 @@ const char* fm_kernel_class_name(uint32_t cls);
  * (a small readback per two rounds, as the plain calls do) and records how
  * many each needed; fm_batch_capture records the whole batch into a CUDA
  * graph with those round counts and no host synchronisation; later
- * fm_batch_run calls replay it.  A replay whose data needs more rounds than
+ * fm_batch_run calls replay it (recording it again first where a larger call
+ * has moved a table's scratch since).  A replay whose data needs more rounds than
  * recorded still gives the same results, more slowly -- run the batch
  * eagerly once on representative data before capturing.  Between
  * fm_batch_run and fm_batch_wait the batch's tables must not be used by other
